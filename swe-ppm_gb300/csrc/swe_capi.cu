@@ -17,6 +17,7 @@
 #include "swe_fast.hpp"
 #include "swe_launch.hpp"
 #include "swe_mlp_launch.hpp"
+#include "swe_sweep.cuh"
 
 
 using namespace swegb;
@@ -146,14 +147,9 @@ __global__ void solveEdgesKernel(long long n, const float *hL, const float *hR, 
     const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float a = hL[i], c = hR[i], e = huL[i], f = huR[i];
-    Cell L, R;
-    L.h = a; L.hn = e; L.b = bL[i];
-    R.h = c; R.hn = f; R.b = bR[i];
-    // per-cell quantities as the sweep kernels form them
-    L.u = (a < kDryTol) ? 0.f : e * (1.f / a);
-    R.u = (c < kDryTol) ? 0.f : f * (1.f / c);
-    L.sq = sqrtf(a); R.sq = sqrtf(c);
-    L.c = kSqrtG * L.sq; R.c = kSqrtG * R.sq;
+    Cell L, R, dummy;
+    cellQuantities<S>(a, e, 0.f, bL[i], L, dummy);
+    cellQuantities<S>(c, f, 0.f, bR[i], R, dummy);
     edgeSolve<S>(L, R, oHL[i], oHR[i], oHuL[i], oHuR[i], oS[i]);
 }
 

@@ -131,17 +131,18 @@ __device__ __forceinline__ float groupTimestep(const DomainDev &d, const GroupSt
 }
 
 /// per-cell quantities in x (normal momentum hu) and y (hv) direction:
-/// u = hu * (1/h), v = hv * (1/h), sqrt(h), sqrt(g) sqrt(h).  Those of a dry
-/// cell are never read (an edge with a dry side solves with the mirrored wet
-/// side), so they are formed without a test.
+/// u = hu * (1/h), v = hv * (1/h), sqrt(h), sqrt(g) sqrt(h) of a tame cell;
+/// sq = -1 marks any other cell, whose derived values are not read
 template <int S> __device__ __forceinline__ void cellQuantities(float h, float hu, float hv, float b, Cell &cx, Cell &cy) {
     float sq = 0.f, c = 0.f, ux = 0.f, uy = 0.f;
     if (S != SOLVER_AUGRIE) {
-        const float rh = 1.f / h;
-        sq = sqrtf(h);
+        const float rh = rcpRn(h);
+        sq = sqrtRn(h);
         if (S == SOLVER_HLLE) c = kSqrtG * sq;
         ux = hu * rh;
         uy = hv * rh;
+        const bool tame = h >= kDryTol && h <= kTameDepth && fabsf(ux) + fabsf(uy) <= kTameSpeed;
+        sq = tame ? sq : -1.f;
     }
     cx = makeCell(h, hu, b, ux, sq, c);
     cy = makeCell(h, hv, b, uy, sq, c);
