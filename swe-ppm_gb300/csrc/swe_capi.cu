@@ -49,39 +49,13 @@ int fail(int code, const char *fmt, ...) {
 // per ghost cell of one block (blockIdx.y); reads touch only interior cells,
 // writes only ghost cells, so blocks never race.
 // ---------------------------------------------------------------------------
-/// mode 0: state ghosts of the groups still stepping; 1: bathymetry ghosts;
-/// 2: the next step's state ghosts of the groups whose update just finished
-/// (ghostsAhead set), as the two-pass update pass pushes them -- the previous
-/// ring stays in the other buffer for downloads; 3: the ring is already the
-/// one mode 0 would write (the update pass pushed it): only hand it to the
-/// current state, as mode 0 does
-__global__ void ghostKernel(const DomainDev d, int mode) {
-    const bool bathymetry = mode == 1;
-    const BlockDesc B = d.blocks[blockIdx.y];
-    const GroupState *G = d.groups + B.group;
-    if ((mode == 0 || mode == 3) && !(*((volatile const float *)&G->time) < *((volatile const float *)&G->target))) return;
-    if (mode == 3) {
-        if (threadIdx.x == 0) const_cast<GroupState *>(G)->ghostsAhead = 0;
-        return;
-    }
-    if (mode == 2 && !*((volatile const int *)&G->ghostsAhead)) return;
-    const int cur = G->cur;
+/// ghost cell i of block B's ring (sides LEFT, RIGHT, BOTTOM, TOP, then the
+/// four corners; past the last: nothing) in nf fields; d.blocks is read only
+/// for CONNECT_WITHIN_RANK sides
+__device__ __forceinline__ void ghostCell(const DomainDev &d, const BlockDesc &B, float *const *fields, int nf,
+                                          bool bathymetry, int i) {
     const int nx = B.nx, ny = B.ny;
     const size_t P = size_t(B.pitch);
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    // the ghost ring of the current buffer now belongs to the current state
-    if (mode == 0 && threadIdx.x == 0) const_cast<GroupState *>(G)->ghostsAhead = 0;
-    float *fields[3];
-    int nf;
-    if (bathymetry) {
-        fields[0] = d.b;
-        nf = 1;
-    } else {
-        fields[0] = cur ? d.h[1] : d.h[0];
-        fields[1] = cur ? d.hu[1] : d.hu[0];
-        fields[2] = cur ? d.hv[1] : d.hv[0];
-        nf = 3;
-    }
     int side, pos;
     if (i < ny) { side = 0; pos = i + 1; }
     else if (i < 2 * ny) { side = 1; pos = i - ny + 1; }
@@ -131,6 +105,40 @@ __global__ void ghostKernel(const DomainDev d, int mode) {
         const float v = fields[f][srcBase + size_t(sx) * srcP + sy];
         fields[f][B.base + size_t(gx) * P + gy] = (negate == f && f > 0) ? -v : v;
     }
+}
+
+/// mode 0: state ghosts of the groups still stepping; 1: bathymetry ghosts;
+/// 2: the next step's state ghosts of the groups whose update just finished
+/// (ghostsAhead set), as the two-pass update pass pushes them -- the previous
+/// ring stays in the other buffer for downloads; 3: the ring is already the
+/// one mode 0 would write (the update pass pushed it): only hand it to the
+/// current state, as mode 0 does
+__global__ void ghostKernel(const DomainDev d, int mode) {
+    const bool bathymetry = mode == 1;
+    const BlockDesc B = d.blocks[blockIdx.y];
+    const GroupState *G = d.groups + B.group;
+    if ((mode == 0 || mode == 3) && !(*((volatile const float *)&G->time) < *((volatile const float *)&G->target))) return;
+    if (mode == 3) {
+        if (threadIdx.x == 0) const_cast<GroupState *>(G)->ghostsAhead = 0;
+        return;
+    }
+    if (mode == 2 && !*((volatile const int *)&G->ghostsAhead)) return;
+    const int cur = G->cur;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    // the ghost ring of the current buffer now belongs to the current state
+    if (mode == 0 && threadIdx.x == 0) const_cast<GroupState *>(G)->ghostsAhead = 0;
+    float *fields[3];
+    int nf;
+    if (bathymetry) {
+        fields[0] = d.b;
+        nf = 1;
+    } else {
+        fields[0] = cur ? d.h[1] : d.h[0];
+        fields[1] = cur ? d.hu[1] : d.hu[0];
+        fields[2] = cur ? d.hv[1] : d.hv[0];
+        nf = 3;
+    }
+    ghostCell(d, B, fields, nf, bathymetry, i);
 }
 
 /// the target time of every group (steps run while time < target)
@@ -2125,25 +2133,17 @@ int noallocScratch(int device, NoAllocScratch **out) {
     return SWE_GPU_OK;
 }
 
-/// writes the block descriptor and work list and clears the control block
-__global__ void noallocSetupKernel(NoAllocScratch *s, BlockDesc b, int tileRows, int tileCols, int nunits) {
+/// writes the block descriptor and work list, clears the control block and
+/// sets the input's ghost ring (setGhostLayer); the ring needs nothing of the
+/// scratch, so one launch does both
+__global__ void noallocSetupKernel(NoAllocScratch *s, DomainDev d, BlockDesc b, int tileRows, int tileCols, int nunits) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i == 0) {
         GroupState g{};
         g.enabled = 1;
-        g.speedBits = 0u;
-        g.arrived = 0u;
         g.units = nunits;
         g.unitsUpd = nunits;
-        g.firstBlock = 0;
-        g.dt = 0.f;
-        g.speed = 0.f;
-        g.time = 0.f;
         g.target = INFINITY;
-        g.steps = 0;
-        g.cur = 0;
-        g.status = 0;
-        g.ghostsAhead = 0;
         s->group = g;
         s->block = b;
     }
@@ -2154,6 +2154,8 @@ __global__ void noallocSetupKernel(NoAllocScratch *s, BlockDesc b, int tileRows,
         s->ctaSeg[u] = u;  // one segment per CTA
     }
     if (i == 0) s->ctaSeg[nunits] = nunits;
+    float *fields[3] = {d.h[0], d.hu[0], d.hv[0]};
+    ghostCell(d, b, fields, 3, false, i);
 }
 
 } // namespace
@@ -2174,14 +2176,22 @@ extern "C" int swe_gpu_step_block_noalloc(int solver, int semantics, int nx, int
         if (boundary[i] < SWE_OUTFLOW || boundary[i] > SWE_PASSIVE || boundary[i] == SWE_CONNECT_WITHIN_RANK)
             return fail(SWE_GPU_ERR_INVALID, "boundary %d: type %d is not valid for a single block", i, boundary[i]);
     const int tileRows = std::min(256, ((ny + 31) / 32) * 32);
-    const int tileCols = 32;
-    const long long nunits = (long long)((ny + tileRows - 1) / tileRows) * ((nx + tileCols - 1) / tileCols);
-    if (nunits > kNoAllocMaxUnits)
+    const long long rowTiles = (ny + tileRows - 1) / tileRows;
+    if (rowTiles * ((nx + 31) / 32) > kNoAllocMaxUnits)
         return fail(SWE_GPU_ERR_INVALID,
                     "block %d x %d needs %lld work units; the allocation-free step supports at most %d "
-                    "(ceil(ny/256) * ceil(nx/32))", nx, ny, nunits, kNoAllocMaxUnits);
-    int device = 0;
+                    "(ceil(ny/256) * ceil(nx/32))", nx, ny, rowTiles * ((nx + 31) / 32), kNoAllocMaxUnits);
+    int device = 0, sms = 148;
     CUDA_TRY(cudaGetDevice(&device));
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    // A segment's columns run one after the other, so a block that does not
+    // fill the GPU gets segments as short as spreads it over all resident
+    // CTAs (4 per SM), down to one column: a 128^2 HLLE step took 75.6 us as 4
+    // segments of 32 columns and takes 20.5 us as 128 of one (host time of
+    // the call included).  Where the GPU is full, segments stay at 32 columns:
+    // shorter ones solve more edges twice.
+    const int tileCols = int(std::max(1LL, std::min(32LL, (rowTiles * nx + 4LL * sms - 1) / (4LL * sms))));
+    const long long nunits = rowTiles * ((nx + tileCols - 1) / tileCols);
     NoAllocScratch *scr = nullptr;
     int rc = noallocScratch(device, &scr);
     if (rc) return rc;
@@ -2223,12 +2233,11 @@ extern "C" int swe_gpu_step_block_noalloc(int solver, int semantics, int nx, int
         g_noallocPtr[device] = nullptr;
         return fail(SWE_GPU_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
     };
-    noallocSetupKernel<<<(unsigned)std::max<long long>(1, std::min<long long>(64, (nunits + 255) / 256)), 256, 0, s>>>(
-        scr, B, tileRows, tileCols, int(nunits));
-    if ((rc = check(cudaGetLastError(), "set-up kernel"))) return rc;
     const int threads = 128;
-    ghostKernel<<<dim3((2 * nx + 2 * ny + 4 + threads - 1) / threads, 1), threads, 0, s>>>(d, 0);
-    if ((rc = check(cudaGetLastError(), "ghost kernel"))) return rc;
+    const long long setupItems = std::max<long long>(2LL * nx + 2LL * ny + 4, nunits);
+    noallocSetupKernel<<<unsigned((setupItems + threads - 1) / threads), threads, 0, s>>>(scr, d, B, tileRows, tileCols,
+                                                                                       int(nunits));
+    if ((rc = check(cudaGetLastError(), "set-up kernel"))) return rc;
     if ((rc = check(launchSpeed(d, int(nunits), tileRows, s), "speed pass"))) return rc;
     if ((rc = check(launchUpdate(d, int(nunits), tileRows, s), "update pass"))) return rc;
     if (dt_out) {
