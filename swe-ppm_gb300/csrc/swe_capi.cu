@@ -581,6 +581,43 @@ struct DomainOptions {
     int ngroups;
 };
 
+/// Rows computed by tiles of TY rows, idle ones of partial tiles included.
+long long paddedRows(const std::vector<BlockDesc> &blocks, int TY) {
+    long long n = 0;
+    for (const BlockDesc &B : blocks) n += (long long)((B.ny + TY - 1) / TY) * TY * B.nx;
+    return n;
+}
+
+/// Default tile height: 256 rows, unless 128-row tiles idle at least 5% fewer
+/// rows.  Where both fill alike, taller tiles solve fewer boundary edges twice
+/// and win by 2-9% (4096^2 as 4 x 4 blocks, fast / exact step: 125 / 231 us
+/// against 128 / 252); partial tiles turn that round (6 x 6 blocks of 300^2,
+/// 1.71 against 1.28 rows per cell: 72 / 87 us against 65 / 75).
+int defaultTileRows(const std::vector<BlockDesc> &blocks) {
+    return paddedRows(blocks, 128) * 20 <= paddedRows(blocks, 256) * 19 ? 128 : 256;
+}
+
+int tileRowsFor(const swe_gpu_domain *D, int arg) {
+    int maxNy = 0;
+    for (const BlockDesc &B : D->blocks) maxNy = std::max(maxNy, B.ny);
+    return std::min(arg > 0 ? arg : defaultTileRows(D->blocks), ((maxNy + 31) / 32) * 32);
+}
+
+/// Cap on the columns per segment: the caller's, else 0 (one run per resident
+/// CTA), else 32 where runs would pass 64 columns and 5% or more of the tiles'
+/// rows are idle.  Equal runs of columns are then unequal work (a run through
+/// a partial tile ends early), and short segments, dealt to CTAs as they
+/// finish, even it out: 128 dam breaks of 64..1024 rows, 637 -> 414 us a fast
+/// step, 702 -> 556 us an exact one (with the tile height above).  Full tiles
+/// gain nothing from it (4096^2: 125 -> 139 us a fast step), and local time
+/// stepping deals its segments out on the device.
+int segmentCap(const swe_gpu_domain *D, int TY, int arg, long long total, long long workers) {
+    if (arg > 0) return arg;
+    long long cells = 0;
+    for (const BlockDesc &B : D->blocks) cells += (long long)B.nx * B.ny;
+    return !D->lts && total > 64 * workers && cells * 20 <= paddedRows(D->blocks, TY) * 19 ? 32 : 0;
+}
+
 /// Balanced persistent partitions of both passes for the domain's current
 /// tile shape; tileColsArg > 0 caps the segment length.
 void buildPartitions(swe_gpu_domain *D, int tileColsArg) {
@@ -602,7 +639,8 @@ void buildPartitions(swe_gpu_domain *D, int tileColsArg) {
         long long total = 0;
         for (const BlockDesc &B : D->blocks) total += (long long)((B.ny + rowsPerTile - 1) / rowsPerTile) * B.nx;
         long long workers = (long long)sms * perSM;
-        if (tileColsArg > 0) workers = std::max(workers, (total + tileColsArg - 1) / tileColsArg);
+        const int segCap = segmentCap(D, rowsPerTile, tileColsArg, total, workers);
+        if (segCap > 0) workers = std::max(workers, (total + segCap - 1) / segCap);
         workers = std::max(1LL, std::min(total, workers));
         std::vector<WorkUnit> &units = pass ? D->unitsU : D->units;
         std::vector<int> &ctaSeg = pass ? D->ctaSegU : D->ctaSeg;
@@ -616,7 +654,7 @@ void buildPartitions(swe_gpu_domain *D, int tileColsArg) {
             while (pos < end) {
                 const BlockDesc &B = D->blocks[k];
                 const long long take = std::min<long long>(end - pos, (long long)(B.nx + 1 - col));
-                const int cap = tileColsArg > 0 ? tileColsArg : kMaxTileCols;
+                const int cap = segCap > 0 ? segCap : kMaxTileCols;
                 const int len = int(std::min<long long>(take, cap));
                 units.push_back(WorkUnit{k, 1 + tile * rowsPerTile, col, col + len});
                 pos += len;
@@ -658,10 +696,11 @@ bool buildFastPlan(swe_gpu_domain *D) {
     long long total = 0;
     for (const BlockDesc &B : D->blocks) total += (long long)((B.ny + TY - 1) / TY) * B.nx;
     long long workers = (long long)sms * occ;
-    if (D->tileColsArg > 0) workers = std::max(workers, (total + D->tileColsArg - 1) / D->tileColsArg);
+    const int segCap = segmentCap(D, TY, D->tileColsArg, total, workers);
+    if (segCap > 0) workers = std::max(workers, (total + segCap - 1) / segCap);
     workers = std::max(1LL, std::min(total, workers));
     D->gridF = int(workers);
-    const int cap = D->tileColsArg > 0 ? std::min(D->tileColsArg, kMaxTileCols) : kMaxTileCols;
+    const int cap = segCap > 0 ? std::min(segCap, kMaxTileCols) : kMaxTileCols;
     D->ctaSegF.assign(1, 0);
     long long pos = 0;
     int k = 0, tile = 0, col = 1;
@@ -789,9 +828,6 @@ int buildDomain(const std::vector<BlockSpec> &spec, const DomainOptions &o, swe_
     D->semantics = o.semantics;
     D->splitDtMode = o.splitDtMode;
     D->tileColsArg = o.tileCols;
-    int maxNy = 0;
-    for (const BlockSpec &b : spec) maxNy = std::max(maxNy, b.ny);
-    D->tileRows = std::min(o.tileRows > 0 ? o.tileRows : 256, ((maxNy + 31) / 32) * 32);
     D->tileCols = o.tileCols > 0 ? o.tileCols : 32;
     const int tileColsArg = o.tileCols;
 
@@ -833,6 +869,7 @@ int buildDomain(const std::vector<BlockSpec> &spec, const DomainOptions &o, swe_
     }
     elems += 32;  // slack so the last column's padding (and the fast step's strip copies) stays inside the allocation
     D->fieldElems = elems;
+    D->tileRows = tileRowsFor(D, o.tileRows);
     buildPartitions(D, tileColsArg);
     D->fast = o.arithmetic == SWE_ARITH_FAST;
     if (D->fast && !buildFastPlan(D)) {
@@ -1689,9 +1726,7 @@ int swe_gpu_retile(swe_gpu_domain *dom, int tile_rows, int tile_cols) {
     if (rc) return rc;
     CUDA_TRY(cudaSetDevice(dom->device));
     CUDA_TRY(cudaStreamSynchronize(dom->stream));
-    int maxNy = 0;
-    for (const BlockDesc &B : dom->blocks) maxNy = std::max(maxNy, B.ny);
-    dom->tileRows = std::min(tile_rows > 0 ? tile_rows : 256, ((maxNy + 31) / 32) * 32);
+    dom->tileRows = tileRowsFor(dom, tile_rows);
     dom->tileColsArg = tile_cols;
     dom->tileCols = tile_cols > 0 ? tile_cols : 32;
     buildPartitions(dom, tile_cols);
