@@ -19,7 +19,7 @@ LIB = os.path.join(OUT, "libswe_gb300.so")
 DRIVER = os.path.join(OUT, "swe_gb300")
 
 CUDA_SOURCES = ["csrc/swe_capi.cu", "csrc/swe_kernels_fh.cu", "csrc/swe_kernels_aug.cu", "csrc/swe_lts.cu", "csrc/swe_mlp.cu",
-                "csrc/swe_fast.cu"]
+                "csrc/swe_fast.cu", "csrc/swe_small.cu"]
 # the fast-arithmetic step (SWE_ARITH_FAST) is its own translation unit with
 # contraction and approximate division and square root
 FAST_SOURCES = {"csrc/swe_fast.cu"}

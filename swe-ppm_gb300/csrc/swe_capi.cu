@@ -17,6 +17,7 @@
 #include "swe_fast.hpp"
 #include "swe_launch.hpp"
 #include "swe_mlp_launch.hpp"
+#include "swe_small.hpp"
 #include "swe_sweep.cuh"
 
 
@@ -251,6 +252,7 @@ struct swe_gpu_domain {
     BlockDesc *dBlocks = nullptr;
     WorkUnit *dUnits = nullptr;
     int *dCtaSeg = nullptr;
+    char *dPlan = nullptr;        // one allocation for dUnits .. dCtaSegU, dUnitsS, dSync
     GroupState *dGroups = nullptr;
     std::vector<int> ctaSeg;      // speed pass: worker c owns segments [ctaSeg[c], ctaSeg[c+1])
     int grid = 0;                 // CTAs of the speed pass
@@ -299,6 +301,14 @@ struct swe_gpu_domain {
     // and applies them (updateUnknowns) instead of solving each edge in both
     // the speed and the update pass
     bool edgeBuffered = false;
+    // small domains (swe_small.cu): several steps per launch, smallCols (0: the
+    // domain is not small) columns per CTA of tileRows rows
+    int speedPassArg = 0;
+    int smallCols = 0;
+    std::vector<WorkUnit> unitsS;
+    std::vector<small::Sync> syncInit;  // one per dt group
+    WorkUnit *dUnitsS = nullptr;
+    small::Sync *dSync = nullptr;
     // asynchronous downloads: two staging slots (4 fields each), copied out on
     // a second stream so one step's download overlaps the next one's upload
     float *stageDown[2] = {nullptr, nullptr};
@@ -332,6 +342,8 @@ struct swe_gpu_domain {
 };
 
 namespace {
+
+constexpr int kSmallSteps = 256;  // steps per launch of a small domain
 
 /// ghost kernel launch; mode as ghostKernel's
 int enqueueGhost(swe_gpu_domain *D, int mode) {
@@ -461,6 +473,28 @@ int enqueueStep(swe_gpu_domain *D) {
     return enqueueUpdate(D);
 }
 
+/// `n` steps; the steps of a small domain in launches of at most 256
+int enqueueSteps(swe_gpu_domain *D, int n) {
+    if (!D->smallCols) {
+        for (int i = 0; i < n; i++) {
+            int rc = enqueueStep(D);
+            if (rc) return rc;
+        }
+        return SWE_GPU_OK;
+    }
+    if (n > 0 && !D->ghostsValid) {
+        int rc = enqueueGhost(D, 0);
+        if (rc) return rc;
+    }
+    for (int done = 0; done < n; done += kSmallSteps) {
+        CUDA_TRY(small::launch(D->dev, D->dUnitsS, int(D->unitsS.size()), D->dSync, std::min(n - done, kSmallSteps),
+                               D->smallCols, D->tileRows, D->stream));
+        D->launches++;
+        D->ghostsValid = true;
+    }
+    return SWE_GPU_OK;
+}
+
 /// one inner iteration of local time stepping (see swe_lts.cu): check
 /// (with the exchange), speed pass of the blocks at an interval start
 /// (unless the check runs it, DomainDev::ltsCheckSpeed), update pass of the
@@ -511,10 +545,7 @@ void freeDomain(swe_gpu_domain *D) {
     cudaFree(D->b);
     cudaFree(D->stage);
     cudaFree(D->dBlocks);
-    cudaFree(D->dUnits);
-    cudaFree(D->dCtaSeg);
-    cudaFree(D->dUnitsU);
-    cudaFree(D->dCtaSegU);
+    cudaFree(D->dPlan);
     cudaFree(D->dUnitsF);
     cudaFree(D->dCtaSegF);
     cudaFree(D->dPieces);
@@ -806,6 +837,69 @@ int uploadFastPlan(swe_gpu_domain *D) {
     return SWE_GPU_OK;
 }
 
+/// Small domains: exact unsplit step with the default segment length, where
+/// segments of 1, 2 or 4 columns cover the domain with CTAs that are resident
+/// together (4 per SM of 256 rows up to 2 columns, 3 at 4).  Step times against
+/// the passes' (us, f-wave and HLLE / hybrid / augmented solver): 256^2 7.2 / 7.7
+/// / 12 against 25 / 17 / 16, 512^2 11 / 11 / - against 24 / 20 / -, 640^2 14 /
+/// 15 / - against 25 / 28 / -.  The augmented solver's edges bound it sooner: at
+/// 2 columns it loses (400^2: 28 against 24).
+void buildSmallPlan(swe_gpu_domain *D) {
+    D->smallCols = 0;
+    D->unitsS.clear();
+    D->syncInit.clear();
+    if (D->fast || D->lts || D->semantics != SEM_UNSPLIT || D->speedPassArg != 0 || D->tileColsArg > 0) return;
+    const int TY = D->tileRows;
+    const int most = D->solver == SOLVER_AUGRIE ? 1 : small::kMaxCols;
+    for (int cols = 1; cols <= most; cols *= 2) {
+        long long n = 0;
+        for (const BlockDesc &B : D->blocks) n += (long long)((B.ny + TY - 1) / TY) * ((B.nx + cols - 1) / cols);
+        if (n > small::capacity(D->solver, cols, TY)) continue;
+        D->smallCols = cols;
+        break;
+    }
+    if (!D->smallCols) return;
+    D->syncInit.assign(D->ngroups, small::Sync{});
+    for (int k = 0; k < int(D->blocks.size()); k++) {
+        const BlockDesc &B = D->blocks[k];
+        small::Sync &y = D->syncInit[B.group];
+        for (int y0 = 1; y0 <= B.ny; y0 += TY)
+            for (int x0 = 1; x0 <= B.nx; x0 += D->smallCols) {
+                if (y.ctas++ == 0) y.first = int(D->unitsS.size());
+                D->unitsS.push_back(WorkUnit{k, y0, x0, std::min(x0 + D->smallCols, B.nx + 1)});
+            }
+    }
+}
+
+/// device copies of the passes' partitions and the small domain's plan, in one
+/// allocation (replacing an earlier one); the meeting points start afresh
+int uploadPlan(swe_gpu_domain *D) {
+    std::vector<char> host;
+    auto put = [&](const void *p, size_t bytes) {
+        const size_t at = (host.size() + 255) / 256 * 256;
+        host.resize(at + bytes);
+        if (bytes) memcpy(host.data() + at, p, bytes);
+        return at;
+    };
+    const size_t oU = put(D->units.data(), sizeof(WorkUnit) * D->units.size());
+    const size_t oC = put(D->ctaSeg.data(), sizeof(int) * D->ctaSeg.size());
+    const size_t oUU = put(D->unitsU.data(), sizeof(WorkUnit) * D->unitsU.size());
+    const size_t oCU = put(D->ctaSegU.data(), sizeof(int) * D->ctaSegU.size());
+    const size_t oS = put(D->unitsS.data(), sizeof(WorkUnit) * D->unitsS.size());
+    const size_t oY = put(D->syncInit.data(), sizeof(small::Sync) * D->syncInit.size());
+    cudaFree(D->dPlan);
+    D->dPlan = nullptr;
+    CUDA_TRY(cudaMalloc(&D->dPlan, host.size() + 256));
+    CUDA_TRY(cudaMemcpy(D->dPlan, host.data(), host.size(), cudaMemcpyHostToDevice));
+    D->dUnits = reinterpret_cast<WorkUnit *>(D->dPlan + oU);
+    D->dCtaSeg = reinterpret_cast<int *>(D->dPlan + oC);
+    D->dUnitsU = reinterpret_cast<WorkUnit *>(D->dPlan + oUU);
+    D->dCtaSegU = reinterpret_cast<int *>(D->dPlan + oCU);
+    D->dUnitsS = reinterpret_cast<WorkUnit *>(D->dPlan + oS);
+    D->dSync = reinterpret_cast<small::Sync *>(D->dPlan + oY);
+    return SWE_GPU_OK;
+}
+
 /// per-group work counts of the passes
 void groupCounts(swe_gpu_domain *D, std::vector<GroupState> &g) {
     for (GroupState &x : g) {
@@ -828,6 +922,7 @@ int buildDomain(const std::vector<BlockSpec> &spec, const DomainOptions &o, swe_
     D->semantics = o.semantics;
     D->splitDtMode = o.splitDtMode;
     D->tileColsArg = o.tileCols;
+    D->speedPassArg = o.speedPass;
     D->tileCols = o.tileCols > 0 ? o.tileCols : 32;
     const int tileColsArg = o.tileCols;
 
@@ -953,10 +1048,6 @@ int buildDomain(const std::vector<BlockSpec> &spec, const DomainOptions &o, swe_
     ok = ok && cudaMalloc(&D->b, bytes) == cudaSuccess;
     ok = ok && cudaMalloc(&D->stage, sizeof(float) * 4 * size_t(D->stageElems)) == cudaSuccess;
     ok = ok && cudaMalloc(&D->dBlocks, sizeof(BlockDesc) * D->blocks.size()) == cudaSuccess;
-    ok = ok && cudaMalloc(&D->dUnits, sizeof(WorkUnit) * D->units.size()) == cudaSuccess;
-    ok = ok && cudaMalloc(&D->dCtaSeg, sizeof(int) * D->ctaSeg.size()) == cudaSuccess;
-    ok = ok && cudaMalloc(&D->dUnitsU, sizeof(WorkUnit) * D->unitsU.size()) == cudaSuccess;
-    ok = ok && cudaMalloc(&D->dCtaSegU, sizeof(int) * D->ctaSegU.size()) == cudaSuccess;
     ok = ok && cudaMalloc(&D->dGroups, sizeof(GroupState) * D->ngroups) == cudaSuccess;
     if (D->lts) {
         ok = ok && cudaMalloc(&D->dLts, sizeof(LtsBlock) * D->blocks.size()) == cudaSuccess;
@@ -994,10 +1085,6 @@ int buildDomain(const std::vector<BlockSpec> &spec, const DomainOptions &o, swe_
     if (D->edgeBuffered && !D->edgeTiles.empty())
         cudaMemcpyAsync(D->dEdgeTiles, D->edgeTiles.data(), sizeof(mlp::EdgeTile) * D->edgeTiles.size(),
                         cudaMemcpyHostToDevice, D->stream);
-    cudaMemcpyAsync(D->dUnits, D->units.data(), sizeof(WorkUnit) * D->units.size(), cudaMemcpyHostToDevice, D->stream);
-    cudaMemcpyAsync(D->dCtaSeg, D->ctaSeg.data(), sizeof(int) * D->ctaSeg.size(), cudaMemcpyHostToDevice, D->stream);
-    cudaMemcpyAsync(D->dUnitsU, D->unitsU.data(), sizeof(WorkUnit) * D->unitsU.size(), cudaMemcpyHostToDevice, D->stream);
-    cudaMemcpyAsync(D->dCtaSegU, D->ctaSegU.data(), sizeof(int) * D->ctaSegU.size(), cudaMemcpyHostToDevice, D->stream);
     cudaMemcpyAsync(D->dGroups, D->groupsInit.data(), sizeof(GroupState) * D->ngroups, cudaMemcpyHostToDevice, D->stream);
     std::vector<LtsBlock> ltsInit;
     LtsControl ctlInit{};
@@ -1035,6 +1122,11 @@ int buildDomain(const std::vector<BlockSpec> &spec, const DomainOptions &o, swe_
             freeDomain(D);
             return rcF;
         }
+    }
+    buildSmallPlan(D);
+    if (const int rcP = uploadPlan(D)) {
+        freeDomain(D);
+        return rcP;
     }
     for (int i = 0; i < 2; i++) {
         D->dev.h[i] = D->h[i];
@@ -1493,11 +1585,7 @@ int swe_gpu_step(swe_gpu_domain *dom, int nsteps) {
     if (dom && dom->lts) return fail(SWE_GPU_ERR_INVALID, "local-time-stepping domain: use swe_gpu_lts_advance");
     if (!dom || nsteps < 0) return fail(SWE_GPU_ERR_INVALID, "bad argument");
     CUDA_TRY(cudaSetDevice(dom->device));
-    for (int i = 0; i < nsteps; i++) {
-        int rc = enqueueStep(dom);
-        if (rc) return rc;
-    }
-    return SWE_GPU_OK;
+    return enqueueSteps(dom, nsteps);
 }
 
 int swe_gpu_advance(swe_gpu_domain *dom, float t_end, int max_steps, int *steps_done, float *t_now) {
@@ -1514,7 +1602,7 @@ int swe_gpu_advance(swe_gpu_domain *dom, float t_end, int max_steps, int *steps_
         CUDA_TRY(cudaStreamBeginCapture(dom->stream, cudaStreamCaptureModeThreadLocal));
         int rc = SWE_GPU_OK;
         const long long before = dom->launches;
-        for (int i = 0; i < batch && rc == SWE_GPU_OK; i++) rc = enqueueStep(dom);
+        rc = enqueueSteps(dom, batch);
         cudaError_t e = cudaStreamEndCapture(dom->stream, &g);
         dom->graphKernels = dom->launches - before;  // captured, not launched
         dom->launches = before;
@@ -1549,10 +1637,8 @@ int swe_gpu_advance(swe_gpu_domain *dom, float t_end, int max_steps, int *steps_
             CUDA_TRY(cudaGraphLaunch(dom->graph, dom->stream));
             dom->launches += dom->graphKernels;
         } else {
-            for (int i = 0; i < remaining; i++) {
-                rc = enqueueStep(dom);
-                if (rc) return rc;
-            }
+            rc = enqueueSteps(dom, remaining);
+            if (rc) return rc;
         }
         rc = readGroups(dom, g);
         if (rc) return rc;
@@ -1568,6 +1654,8 @@ int swe_gpu_advance(swe_gpu_domain *dom, float t_end, int max_steps, int *steps_
         status |= x.status;
     }
     if (t_now) *t_now = tmin;
+    if (dom->smallCols && (status & 8))  // a wait ran out: the meeting points start afresh
+        CUDA_TRY(cudaMemcpy(dom->dSync, dom->syncInit.data(), sizeof(small::Sync) * dom->syncInit.size(), cudaMemcpyHostToDevice));
     if (status) return fail(SWE_GPU_ERR_DEVICE, "device status 0x%x (NaN wave speed)", status);
     return SWE_GPU_OK;
 }
@@ -1730,23 +1818,9 @@ int swe_gpu_retile(swe_gpu_domain *dom, int tile_rows, int tile_cols) {
     dom->tileColsArg = tile_cols;
     dom->tileCols = tile_cols > 0 ? tile_cols : 32;
     buildPartitions(dom, tile_cols);
-    // device copies of the new partitions; per-group segment counts
-    cudaFree(dom->dUnits);
-    cudaFree(dom->dCtaSeg);
-    cudaFree(dom->dUnitsU);
-    cudaFree(dom->dCtaSegU);
-    dom->dUnits = nullptr;
-    dom->dCtaSeg = nullptr;
-    dom->dUnitsU = nullptr;
-    dom->dCtaSegU = nullptr;
-    CUDA_TRY(cudaMalloc(&dom->dUnits, sizeof(WorkUnit) * dom->units.size()));
-    CUDA_TRY(cudaMalloc(&dom->dCtaSeg, sizeof(int) * dom->ctaSeg.size()));
-    CUDA_TRY(cudaMalloc(&dom->dUnitsU, sizeof(WorkUnit) * dom->unitsU.size()));
-    CUDA_TRY(cudaMalloc(&dom->dCtaSegU, sizeof(int) * dom->ctaSegU.size()));
-    CUDA_TRY(cudaMemcpy(dom->dUnits, dom->units.data(), sizeof(WorkUnit) * dom->units.size(), cudaMemcpyHostToDevice));
-    CUDA_TRY(cudaMemcpy(dom->dCtaSeg, dom->ctaSeg.data(), sizeof(int) * dom->ctaSeg.size(), cudaMemcpyHostToDevice));
-    CUDA_TRY(cudaMemcpy(dom->dUnitsU, dom->unitsU.data(), sizeof(WorkUnit) * dom->unitsU.size(), cudaMemcpyHostToDevice));
-    CUDA_TRY(cudaMemcpy(dom->dCtaSegU, dom->ctaSegU.data(), sizeof(int) * dom->ctaSegU.size(), cudaMemcpyHostToDevice));
+    buildSmallPlan(dom);
+    if ((rc = uploadPlan(dom))) return rc;
+    // per-group segment counts
     std::vector<GroupState> g;
     rc = readGroups(dom, g);
     if (rc) return rc;
@@ -1850,9 +1924,9 @@ int swe_gpu_autotune(swe_gpu_domain *dom, int trial_steps, int *best_rows, int *
         for (int c : colCands) {
             if ((rc = swe_gpu_retile(dom, r, c))) break;
             if ((e = copyState(false)) != cudaSuccess) break;
-            for (int i = 0; i < 2 && !rc; i++) rc = enqueueStep(dom);  // warm-up
+            rc = enqueueSteps(dom, 2);  // warm-up
             cudaEventRecord(e0, dom->stream);
-            for (int i = 0; i < trial_steps && !rc; i++) rc = enqueueStep(dom);
+            if (!rc) rc = enqueueSteps(dom, trial_steps);
             cudaEventRecord(e1, dom->stream);
             if (rc || (e = cudaEventSynchronize(e1)) != cudaSuccess) break;
             float ms = 0.f;

@@ -1,0 +1,34 @@
+// Several time steps of a small domain in one cooperative launch
+// (swe_small.cu), called by the domain entry points of swe_capi.cu.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include "swe_device.cuh"
+
+namespace swegb {
+namespace small {
+
+/// Meeting point of a dt group's CTAs, zero before the first launch; every
+/// meeting leaves count at 0 and speed at 0.
+struct __align__(128) Sync {
+    unsigned count;            // CTAs that have arrived
+    unsigned speed;            // the step's largest wave speed so far (float bits)
+    unsigned long long epoch;  // (meetings so far << 32) | dt bits of the last one that formed a dt
+    int ctas;                  // CTAs of the group
+    int first;                 // the group's first CTA (publishes the clock)
+};
+
+constexpr int kMaxCols = 4;  // most columns of a CTA's segment
+
+/// CTAs of `threads` rows and up to `cols` columns (1, 2 or 4) that are
+/// resident at once on the current device; 0 when it cannot launch them together
+int capacity(int solver, int cols, int threads);
+
+/// up to nsteps unsplit steps of every group that has not reached its target
+/// (fewer once it has); units[i] is CTA i's segment of at most `cols` columns
+cudaError_t launch(const DomainDev &d, const WorkUnit *units, int nunits, Sync *sync, int nsteps, int cols, int threads,
+                   cudaStream_t s);
+
+} // namespace small
+} // namespace swegb
