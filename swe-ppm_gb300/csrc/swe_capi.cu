@@ -235,6 +235,8 @@ __global__ void snapshotKernel(const DomainDev d, int k, uint32_t *out) {
 
 } // namespace
 
+constexpr int kAdvanceAhead = 4;  // batches of steps swe_gpu_advance keeps in flight
+
 struct swe_gpu_domain {
     int device = 0;
     cudaStream_t stream = nullptr;     // stream launches go to
@@ -268,6 +270,12 @@ struct swe_gpu_domain {
     int maxCols = 0;              // max nx+2 over blocks
     cudaGraphExec_t graph = nullptr;
     int graphSteps = 0;
+    // swe_gpu_advance: the groups' states at its start and after each batch of
+    // steps in flight (pinned), the events that mark their copies, and the
+    // clock and dt it saw last
+    GroupState *groupsHost = nullptr;
+    cudaEvent_t groupsReady[kAdvanceAhead + 1] = {};
+    float hintTime = 0.f, hintDt = 0.f;
     cudaEvent_t snapEvent = nullptr;  // completion of the last snapshot copy
     bool bounded = false;             // bounded speed pass (f-wave / HLLE, unsplit, CTA tiles)
     std::vector<TileInfo> tiles;      // bound tiles of all blocks
@@ -521,7 +529,6 @@ int readGroups(swe_gpu_domain *D, std::vector<GroupState> &g) {
 int setTargets(swe_gpu_domain *D, float target) {
     setTargetsKernel<<<(D->ngroups + 255) / 256, 256, 0, D->stream>>>(D->dGroups, D->ngroups, target);
     CUDA_TRY(cudaGetLastError());
-    CUDA_TRY(cudaStreamSynchronize(D->stream));
     return SWE_GPU_OK;
 }
 
@@ -534,6 +541,9 @@ void freeDomain(swe_gpu_domain *D) {
     cudaFree(D->dLtsLocal);
     for (int f = 0; f < 3; f++) cudaFree(D->dRing[f]);
     if (D->ltsCtlHost) cudaFreeHost(D->ltsCtlHost);
+    if (D->groupsHost) cudaFreeHost(D->groupsHost);
+    for (cudaEvent_t ev : D->groupsReady)
+        if (ev) cudaEventDestroy(ev);
     for (int j = 0; j < 2; j++)
         if (D->ltsCtlReady[j]) cudaEventDestroy(D->ltsCtlReady[j]);
     if (D->snapEvent) cudaEventDestroy(D->snapEvent);
@@ -1613,45 +1623,86 @@ int swe_gpu_advance(swe_gpu_domain *dom, float t_end, int max_steps, int *steps_
         if (e != cudaSuccess) return fail(SWE_GPU_ERR_CUDA, "graph instantiate: %s", cudaGetErrorString(e));
         dom->graphSteps = batch;
     }
-    std::vector<GroupState> g;
-    int rc = readGroups(dom, g);
+    if (!dom->groupsHost) {
+        cudaError_t e = cudaMallocHost(&dom->groupsHost, sizeof(GroupState) * dom->ngroups * (kAdvanceAhead + 1));
+        if (e != cudaSuccess) {
+            dom->groupsHost = nullptr;
+            return fail(SWE_GPU_ERR_NOMEM, "cudaMallocHost: %s", cudaGetErrorString(e));
+        }
+        for (cudaEvent_t &ev : dom->groupsReady) CUDA_TRY(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+    }
+    // The groups' clocks come back in stream order, one copy per batch of
+    // steps, so the device need not wait for the host between batches: the next
+    // ones are queued while the last step's dt says that they will be needed
+    // (steps queued past t_end do nothing).  Waiting for each batch cost 15 to
+    // 20 us apiece.
+    auto copyGroups = [&](int slot) -> int {
+        CUDA_TRY(cudaMemcpyAsync(dom->groupsHost + size_t(slot) * dom->ngroups, dom->dGroups, sizeof(GroupState) * dom->ngroups,
+                                 cudaMemcpyDeviceToHost, dom->stream));
+        CUDA_TRY(cudaEventRecord(dom->groupsReady[slot], dom->stream));
+        return SWE_GPU_OK;
+    };
+    const int ng = dom->ngroups, startSlot = kAdvanceAhead;
+    int rc = copyGroups(startSlot);
     if (rc) return rc;
-    std::vector<int> startSteps(g.size());
-    for (size_t i = 0; i < g.size(); i++) startSteps[i] = g[i].steps;
     rc = setTargets(dom, t_end);
     if (rc) return rc;
-    // steps taken (the most any group took) and whether every group reached t_end
-    auto progress = [&](int &steps) {
-        steps = 0;
-        bool all = true;
-        for (size_t i = 0; i < g.size(); i++) {
-            steps = std::max(steps, g[i].steps - startSteps[i]);
-            all = all && !(g[i].time < t_end);
-        }
-        return all;
-    };
-    int done = 0;
-    while (done < max_steps) {
-        const int remaining = max_steps - done;
-        if (remaining >= dom->graphSteps) {
-            CUDA_TRY(cudaGraphLaunch(dom->graph, dom->stream));
-            dom->launches += dom->graphKernels;
-        } else {
-            rc = enqueueSteps(dom, remaining);
+    const GroupState *g = dom->groupsHost + size_t(startSlot) * ng, *start = g;
+    int done = 0, queued = 0, ahead = 0, oldest = 0;  // batches in slots oldest .. oldest + ahead - 1
+    float seenTime = dom->hintTime, seenDt = dom->hintDt;  // of the last batch read (a hint: other calls may have moved the clock)
+    int seenQueued = 0;                                    // steps queued up to it
+    int sizes[kAdvanceAhead];
+    bool all = false;
+    while (!all && (ahead > 0 || done < max_steps)) {
+        while (queued < max_steps && ahead < kAdvanceAhead &&
+               (ahead == 0 || double(seenTime) + double(seenDt) * (queued - seenQueued) < double(t_end))) {
+            if (ahead > 0 && !(seenDt > 0.f)) break;
+            const int n = std::min(max_steps - queued, dom->graphSteps);
+            if (n == dom->graphSteps) {
+                CUDA_TRY(cudaGraphLaunch(dom->graph, dom->stream));
+                dom->launches += dom->graphKernels;
+            } else {
+                rc = enqueueSteps(dom, n);
+                if (rc) return rc;
+            }
+            const int slot = (oldest + ahead) % kAdvanceAhead;
+            rc = copyGroups(slot);
             if (rc) return rc;
+            sizes[slot] = n;
+            queued += n;
+            ahead++;
         }
-        rc = readGroups(dom, g);
-        if (rc) return rc;
-        if (progress(done)) break;
+        if (ahead == 0) break;
+        CUDA_TRY(cudaEventSynchronize(dom->groupsReady[oldest]));
+        g = dom->groupsHost + size_t(oldest) * ng;
+        seenQueued += sizes[oldest];
+        oldest = (oldest + 1) % kAdvanceAhead;
+        ahead--;
+        // steps taken (the most any group took) and whether every group reached t_end
+        done = 0;
+        all = true;
+        seenTime = INFINITY;
+        seenDt = 0.f;
+        for (int i = 0; i < ng; i++) {
+            done = std::max(done, g[i].steps - start[i].steps);
+            all = all && !(g[i].time < t_end);
+            if (g[i].time < seenTime) {
+                seenTime = g[i].time;
+                seenDt = g[i].dt;
+            }
+        }
     }
+    dom->hintTime = seenTime;
+    dom->hintDt = seenDt;
+    if (queued == 0) CUDA_TRY(cudaEventSynchronize(dom->groupsReady[startSlot]));
     rc = setTargets(dom, INFINITY);
     if (rc) return rc;
     if (steps_done) *steps_done = done;
     float tmin = g[0].time;
     int status = 0;
-    for (const GroupState &x : g) {
-        tmin = std::min(tmin, x.time);
-        status |= x.status;
+    for (int i = 0; i < ng; i++) {
+        tmin = std::min(tmin, g[i].time);
+        status |= g[i].status;
     }
     if (t_now) *t_now = tmin;
     if (dom->smallCols && (status & 8))  // a wait ran out: the meeting points start afresh
