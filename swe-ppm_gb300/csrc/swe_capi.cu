@@ -392,6 +392,11 @@ int enqueueSpeed(swe_gpu_domain *D) {
         D->launches++;
         return SWE_GPU_OK;
     }
+    if (D->semantics == SEM_SPLIT && D->splitDtMode == SPLIT_DT_LAST_EDGE) {
+        CUDA_TRY(launchLastEdge(d, D->ngroups, D->stream));
+        D->launches++;
+        return SWE_GPU_OK;
+    }
     d.units = D->dUnits;
     d.ctaSeg = D->dCtaSeg;
     // local time stepping: most iterations list no block for the speed pass
@@ -403,7 +408,8 @@ int enqueueSpeed(swe_gpu_domain *D) {
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, D->device);
         grid = std::min(grid, 2 * sms);
     }
-    CUDA_TRY(launchSpeed(d, grid, D->tileRows, D->stream));
+    // (its early start would delay the update's there, so it launches plainly)
+    CUDA_TRY(launchSpeed(d, grid, D->tileRows, D->stream, !D->lts));
     D->launches++;
     return SWE_GPU_OK;
 }
@@ -456,7 +462,7 @@ int enqueueFastPrologue(swe_gpu_domain *D) {
         DomainDev d = D->dev;
         d.units = D->dUnits;
         d.ctaSeg = D->dCtaSeg;
-        CUDA_TRY(launchSpeed(d, D->grid, D->tileRows, D->stream));
+        CUDA_TRY(launchSpeed(d, D->grid, D->tileRows, D->stream, true));
         D->launches++;
         D->dtValid = true;
     }
@@ -2398,7 +2404,7 @@ extern "C" int swe_gpu_step_block_noalloc(int solver, int semantics, int nx, int
     noallocSetupKernel<<<unsigned((setupItems + threads - 1) / threads), threads, 0, s>>>(scr, d, B, tileRows, tileCols,
                                                                                        int(nunits));
     if ((rc = check(cudaGetLastError(), "set-up kernel"))) return rc;
-    if ((rc = check(launchSpeed(d, int(nunits), tileRows, s), "speed pass"))) return rc;
+    if ((rc = check(launchSpeed(d, int(nunits), tileRows, s, false), "speed pass"))) return rc;
     if ((rc = check(launchUpdate(d, int(nunits), tileRows, s), "update pass"))) return rc;
     if (dt_out) {
         if ((rc = check(cudaMemcpyAsync(dt_out, &scr->group.dt, sizeof(float), cudaMemcpyDeviceToHost, s), "dt copy")))

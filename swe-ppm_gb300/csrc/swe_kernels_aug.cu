@@ -5,23 +5,25 @@
 
 namespace swegb {
 
-template <int S> static cudaError_t speed(const DomainDev &d, int n, int th, cudaStream_t s) {
-    if (d.semantics == SEM_SPLIT)
-        speedSplitKernel<S><<<n, th, 0, s>>>(d);
-    else
-        sweepKernel<S, SEM_UNSPLIT, false><<<n, th, 0, s>>>(d);
+template <int S> static cudaError_t speed(const DomainDev &d, int n, int th, cudaStream_t s, bool pdl) {
+    const auto k = d.semantics == SEM_SPLIT ? speedSplitKernel<S> : sweepKernel<S, SEM_UNSPLIT, false>;
+    if (pdl) return launchPdl(k, dim3(n), dim3(th), s, d);
+    k<<<n, th, 0, s>>>(d);
     return cudaGetLastError();
 }
 template <int S> static cudaError_t update(const DomainDev &d, int n, int th, cudaStream_t s) {
-    if (d.semantics == SEM_SPLIT)
-        sweepKernel<S, SEM_SPLIT, true><<<n, th, 0, s>>>(d);
-    else
-        sweepKernel<S, SEM_UNSPLIT, true><<<n, th, 0, s>>>(d);
-    return cudaGetLastError();
+    return d.semantics == SEM_SPLIT ? launchPdl(sweepKernel<S, SEM_SPLIT, true>, dim3(n), dim3(th), s, d)
+                                    : launchPdl(sweepKernel<S, SEM_UNSPLIT, true>, dim3(n), dim3(th), s, d);
+}
+template <int S> static cudaError_t lastEdge(const DomainDev &d, int ngroups, cudaStream_t s) {
+    return launchPdl(lastEdgeKernel<S>, dim3((ngroups + 31) / 32), dim3(32), s, d, ngroups);
 }
 
-cudaError_t launchSpeedAug(const DomainDev &d, int n, int th, cudaStream_t s) {
-    return d.solver == SOLVER_AUGRIE ? speed<SOLVER_AUGRIE>(d, n, th, s) : speed<SOLVER_HYBRID>(d, n, th, s);
+cudaError_t launchSpeedAug(const DomainDev &d, int n, int th, cudaStream_t s, bool pdl) {
+    return d.solver == SOLVER_AUGRIE ? speed<SOLVER_AUGRIE>(d, n, th, s, pdl) : speed<SOLVER_HYBRID>(d, n, th, s, pdl);
+}
+cudaError_t launchLastEdgeAug(const DomainDev &d, int ngroups, cudaStream_t s) {
+    return d.solver == SOLVER_AUGRIE ? lastEdge<SOLVER_AUGRIE>(d, ngroups, s) : lastEdge<SOLVER_HYBRID>(d, ngroups, s);
 }
 cudaError_t launchUpdateAug(const DomainDev &d, int n, int th, cudaStream_t s) {
     return d.solver == SOLVER_AUGRIE ? update<SOLVER_AUGRIE>(d, n, th, s) : update<SOLVER_HYBRID>(d, n, th, s);

@@ -5,25 +5,25 @@
 
 namespace swegb {
 
-template <int S> static cudaError_t speed(const DomainDev &d, int n, int th, cudaStream_t s) {
-    if (d.semantics == SEM_SPLIT)
-        speedSplitKernel<S><<<n, th, 0, s>>>(d);
-    else
-        sweepKernel<S, SEM_UNSPLIT, false><<<n, th, 0, s>>>(d);
+template <int S> static cudaError_t speed(const DomainDev &d, int n, int th, cudaStream_t s, bool pdl) {
+    const auto k = d.semantics == SEM_SPLIT ? speedSplitKernel<S> : sweepKernel<S, SEM_UNSPLIT, false>;
+    if (pdl) return launchPdl(k, dim3(n), dim3(th), s, d);
+    k<<<n, th, 0, s>>>(d);
     return cudaGetLastError();
 }
 template <int S> static cudaError_t update(const DomainDev &d, int n, int th, cudaStream_t s) {
-    if (d.semantics == SEM_SPLIT) {
-        sweepKernel<S, SEM_SPLIT, true><<<n, th, 0, s>>>(d);
-    } else {
-        cudaError_t e = launchPdl(sweepKernel<S, SEM_UNSPLIT, true>, dim3(n), dim3(th), s, d);
-        if (e != cudaSuccess) return e;
-    }
-    return cudaGetLastError();
+    return d.semantics == SEM_SPLIT ? launchPdl(sweepKernel<S, SEM_SPLIT, true>, dim3(n), dim3(th), s, d)
+                                    : launchPdl(sweepKernel<S, SEM_UNSPLIT, true>, dim3(n), dim3(th), s, d);
+}
+template <int S> static cudaError_t lastEdge(const DomainDev &d, int ngroups, cudaStream_t s) {
+    return launchPdl(lastEdgeKernel<S>, dim3((ngroups + 31) / 32), dim3(32), s, d, ngroups);
 }
 
-cudaError_t launchSpeedFH(const DomainDev &d, int n, int th, cudaStream_t s) {
-    return d.solver == SOLVER_FWAVE ? speed<SOLVER_FWAVE>(d, n, th, s) : speed<SOLVER_HLLE>(d, n, th, s);
+cudaError_t launchSpeedFH(const DomainDev &d, int n, int th, cudaStream_t s, bool pdl) {
+    return d.solver == SOLVER_FWAVE ? speed<SOLVER_FWAVE>(d, n, th, s, pdl) : speed<SOLVER_HLLE>(d, n, th, s, pdl);
+}
+cudaError_t launchLastEdgeFH(const DomainDev &d, int ngroups, cudaStream_t s) {
+    return d.solver == SOLVER_FWAVE ? lastEdge<SOLVER_FWAVE>(d, ngroups, s) : lastEdge<SOLVER_HLLE>(d, ngroups, s);
 }
 cudaError_t launchUpdateFH(const DomainDev &d, int n, int th, cudaStream_t s) {
     return d.solver == SOLVER_FWAVE ? update<SOLVER_FWAVE>(d, n, th, s) : update<SOLVER_HLLE>(d, n, th, s);

@@ -43,12 +43,17 @@ inline cudaError_t launchPdlSmem(void (*k)(P...), dim3 grid, dim3 block, size_t 
 }
 
 // speed pass (computeNumericalFluxes' wave speeds + maxTimestep) and fused
-// solve-and-update pass (updateUnknowns) of the f-wave and HLLE solvers
-cudaError_t launchSpeedFH(const DomainDev &d, int nunits, int threads, cudaStream_t s);
+// solve-and-update pass (updateUnknowns) of the f-wave and HLLE solvers.
+// pdl: the speed pass may be scheduled while the previous kernel finishes; the
+// work list must then be one that no kernel in flight writes
+cudaError_t launchSpeedFH(const DomainDev &d, int nunits, int threads, cudaStream_t s, bool pdl);
 cudaError_t launchUpdateFH(const DomainDev &d, int nunits, int threads, cudaStream_t s);
+// the split step's dt from its last x-edge (SPLIT_DT_LAST_EDGE)
+cudaError_t launchLastEdgeFH(const DomainDev &d, int ngroups, cudaStream_t s);
 // same for the augmented and hybrid solvers
-cudaError_t launchSpeedAug(const DomainDev &d, int nunits, int threads, cudaStream_t s);
+cudaError_t launchSpeedAug(const DomainDev &d, int nunits, int threads, cudaStream_t s, bool pdl);
 cudaError_t launchUpdateAug(const DomainDev &d, int nunits, int threads, cudaStream_t s);
+cudaError_t launchLastEdgeAug(const DomainDev &d, int ngroups, cudaStream_t s);
 
 // bounded speed pass of the f-wave and HLLE unsplit step over the bound
 // tiles (d.tileInfo, d.tileW, d.tileKey), 256 threads per CTA
@@ -72,9 +77,13 @@ inline int passOccupancy(int solver, int sem, bool update, int threads) {
                                                            : occupancyAug(solver, sem, update, threads);
 }
 
-inline cudaError_t launchSpeed(const DomainDev &d, int nunits, int threads, cudaStream_t s) {
-    return (d.solver == SOLVER_FWAVE || d.solver == SOLVER_HLLE) ? launchSpeedFH(d, nunits, threads, s)
-                                                                 : launchSpeedAug(d, nunits, threads, s);
+inline cudaError_t launchSpeed(const DomainDev &d, int nunits, int threads, cudaStream_t s, bool pdl) {
+    return (d.solver == SOLVER_FWAVE || d.solver == SOLVER_HLLE) ? launchSpeedFH(d, nunits, threads, s, pdl)
+                                                                 : launchSpeedAug(d, nunits, threads, s, pdl);
+}
+inline cudaError_t launchLastEdge(const DomainDev &d, int ngroups, cudaStream_t s) {
+    return (d.solver == SOLVER_FWAVE || d.solver == SOLVER_HLLE) ? launchLastEdgeFH(d, ngroups, s)
+                                                                 : launchLastEdgeAug(d, ngroups, s);
 }
 inline cudaError_t launchUpdate(const DomainDev &d, int nunits, int threads, cudaStream_t s) {
     return (d.solver == SOLVER_FWAVE || d.solver == SOLVER_HLLE) ? launchUpdateFH(d, nunits, threads, s)

@@ -269,6 +269,17 @@ __device__ __forceinline__ void ltsEndIteration(const DomainDev &d) {
     }
 }
 
+/// speed of the last x-edge the serial split loop solves, (nx | nx+1) in row
+/// ny+1: all that its dt keeps (SPLIT_DT_LAST_EDGE)
+template <int S> __device__ __forceinline__ float lastEdgeSpeed(const DomainDev &d, const BlockDesc &F, int cur) {
+    const float *H = pick(d.h, cur) + F.base, *HU = pick(d.hu, cur) + F.base, *BT = d.b + F.base;
+    const size_t o = size_t(F.nx) * size_t(F.pitch) + size_t(F.ny + 1), o2 = o + size_t(F.pitch);
+    Cell L, R, dummy;
+    cellQuantities<S>(H[o], HU[o], 0.f, BT[o], L, dummy);
+    cellQuantities<S>(H[o2], HU[o2], 0.f, BT[o2], R, dummy);
+    return vmax(0.f, edgeSpeed<S>(L, R));
+}
+
 /// the segment's share of the running pass is done; the last segment of the
 /// group finishes the pass (dt after the speed pass; clock, step count and
 /// current buffer after the update pass)
@@ -304,36 +315,6 @@ __device__ __forceinline__ void segmentDone(const DomainDev &d, GroupState *G, f
         } else {
             float s = __uint_as_float(__ldcg(&G->speedBits));  // every CTA's maximum (acquired above)
             const BlockDesc &F = d.blocks[G->firstBlock];
-            if (d.semantics == SEM_SPLIT && d.splitDtMode == SPLIT_DT_LAST_EDGE) {
-                // speed of the last x-edge the serial loop solves: (nx | nx+1) in row ny+1
-                const float *Hc = pick(d.h, cur) + F.base, *HUc = pick(d.hu, cur) + F.base, *Bc = d.b + F.base;
-                const size_t o = size_t(F.nx) * size_t(F.pitch) + size_t(F.ny + 1);
-                const size_t o2 = o + size_t(F.pitch);
-                Cell L, R, dummy;
-                switch (d.solver) {
-                case SOLVER_FWAVE:
-                    cellQuantities<SOLVER_FWAVE>(Hc[o], HUc[o], 0.f, Bc[o], L, dummy);
-                    cellQuantities<SOLVER_FWAVE>(Hc[o2], HUc[o2], 0.f, Bc[o2], R, dummy);
-                    s = edgeSpeed<SOLVER_FWAVE>(L, R);
-                    break;
-                case SOLVER_HLLE:
-                    cellQuantities<SOLVER_HLLE>(Hc[o], HUc[o], 0.f, Bc[o], L, dummy);
-                    cellQuantities<SOLVER_HLLE>(Hc[o2], HUc[o2], 0.f, Bc[o2], R, dummy);
-                    s = edgeSpeed<SOLVER_HLLE>(L, R);
-                    break;
-                case SOLVER_AUGRIE:
-                    cellQuantities<SOLVER_AUGRIE>(Hc[o], HUc[o], 0.f, Bc[o], L, dummy);
-                    cellQuantities<SOLVER_AUGRIE>(Hc[o2], HUc[o2], 0.f, Bc[o2], R, dummy);
-                    s = edgeSpeed<SOLVER_AUGRIE>(L, R);
-                    break;
-                default:
-                    cellQuantities<SOLVER_HYBRID>(Hc[o], HUc[o], 0.f, Bc[o], L, dummy);
-                    cellQuantities<SOLVER_HYBRID>(Hc[o2], HUc[o2], 0.f, Bc[o2], R, dummy);
-                    s = edgeSpeed<SOLVER_HYBRID>(L, R);
-                    break;
-                }
-                s = vmax(0.f, s);
-            }
             G->speed = s;
             G->dt = groupTimestep(d, G, s, F.dx, F.dy);
             if (!(s == s)) G->status |= 1;  // NaN wave speed
@@ -730,6 +711,7 @@ __global__ void __launch_bounds__(kMaxTileRows, 4) sweepKernel(const DomainDev d
 template <int S> __global__ void __launch_bounds__(kMaxTileRows) speedSplitKernel(const DomainDev d) {
     __shared__ float sRed[kMaxTileRows / 32];
     __shared__ int sLast;
+    pdlWaitAndRelease();
     const int TY = blockDim.x;
     const int segEnd = d.ctaSeg[blockIdx.x + 1];
     for (int seg = d.ctaSeg[blockIdx.x]; seg < segEnd; ++seg) {
@@ -762,6 +744,27 @@ template <int S> __global__ void __launch_bounds__(kMaxTileRows) speedSplitKerne
         }
         segmentDone<false>(d, G, smax, sRed, &sLast, cur);
     }
+}
+
+/// the split block's dt where it keeps only the last edge's speed
+/// (src/blocks/SWE_DimensionalSplitting.cpp:131-136): that one edge instead of a
+/// pass over all of them, whose maximum nothing reads.  One thread per group;
+/// latency alone (about 3 us of a launch against 17 us for the pass at
+/// 1021 x 2039).
+template <int S> __global__ void lastEdgeKernel(const DomainDev d, int ngroups) {
+    // the update pass may take its place on the SMs at once: it waits for this
+    // grid, which waits for the one before
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int g = blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= ngroups) return;
+    GroupState *G = d.groups + g;
+    if (!groupActive(G)) return;
+    const BlockDesc &F = d.blocks[G->firstBlock];
+    const float s = lastEdgeSpeed<S>(d, F, G->cur);
+    G->speed = s;
+    G->dt = timestepFromSpeed(s, F.dx, F.dy, SEM_SPLIT);
+    if (!(s == s)) G->status |= 1;  // NaN wave speed
 }
 
 } // namespace swegb
