@@ -68,8 +68,15 @@ __device__ void randomEdge(uint64_t i, float e[6]) {
     if (kind < 6) e[3] = e[2] * (1.f + 0.1f * (u() - 0.5f));
     e[4] = -e[0] * (0.5f + u());
     e[5] = kind % 2 ? e[4] + (e[0] - e[1]) * (u() < 0.5f ? 1.f : u()) : -e[1] * (0.5f + u());
-    if (kind == 6) e[2] *= exp2f(-100.f * u());
-    if (kind == 7) e[3] *= exp2f(-100.f * u());
+    if (kind == 6) e[2] *= exp2f(-140.f * u());
+    if (kind == 7) {
+        e[3] *= exp2f(-140.f * u());
+        if (u() < 0.5f) {  // still water over a flat or uneven bed
+            e[1] = e[0];
+            e[2] = e[3] * u();
+            e[5] = u() < 0.5f ? e[4] : e[4] * (1.f + exp2f(-22.f));
+        }
+    }
     if (kind == 8) e[2] = u() < 0.5f ? 0.f : -0.f;
     if (kind == 9) e[3] = u() < 0.5f ? 0.f : -0.f;
     if (kind == 8 || kind == 9) e[5] = e[4];
