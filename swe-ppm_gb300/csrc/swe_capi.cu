@@ -300,8 +300,8 @@ struct swe_gpu_domain {
     LtsControl *ltsCtlHost = nullptr;
     cudaEvent_t ltsCtlReady[2] = {nullptr, nullptr};
     // surrogate step and edge logger: edge tiles and the stored net updates
-    std::vector<mlp::EdgeTile> edgeTiles;
-    mlp::EdgeTile *dEdgeTiles = nullptr;
+    std::vector<mlp::EdgeTile> edgeTiles, stepTiles;  // the logger's, the edge pass's
+    mlp::EdgeTile *dEdgeTiles = nullptr, *dStepTiles = nullptr;
     float *edgeBuf = nullptr;             // 8 fields: x-edge then y-edge net updates
     unsigned long long *dUsed = nullptr;  // edges the surrogate solved
     // augmented solver, unsplit, CTA tiles, global time stepping: the step
@@ -381,7 +381,7 @@ long long maxBlockCells(const swe_gpu_domain *D) {
 int enqueueSpeed(swe_gpu_domain *D) {
     DomainDev d = D->dev;
     if (D->edgeBuffered) {
-        CUDA_TRY(mlp::launchSurrogateEdges(d, nullptr, D->dEdgeTiles, int(D->edgeTiles.size()), edgeUpdates(D), D->dUsed,
+        CUDA_TRY(mlp::launchSurrogateEdges(d, nullptr, D->dStepTiles, int(D->stepTiles.size()), edgeUpdates(D), D->dUsed,
                                            D->stream));
         CUDA_TRY(mlp::launchSurrogateDt(d, D->ngroups, D->stream));
         D->launches += 2;
@@ -572,6 +572,7 @@ void freeDomain(swe_gpu_domain *D) {
     cudaFree(D->dTileW);
     cudaFree(D->dTileKey);
     cudaFree(D->dEdgeTiles);
+    cudaFree(D->dStepTiles);
     cudaFree(D->edgeBuf);
     cudaFree(D->dUsed);
     for (int j = 0; j < 2; j++) {
@@ -1076,10 +1077,10 @@ int buildDomain(const std::vector<BlockSpec> &spec, const DomainOptions &o, swe_
     D->edgeBuffered = D->solver == SOLVER_AUGRIE && D->semantics == SEM_UNSPLIT && !D->lts &&
                       o.speedPass == 0;
     if (D->edgeBuffered) {
-        D->edgeTiles = mlp::buildEdgeTiles(D->blocks);
+        D->stepTiles = mlp::buildStepTiles(D->blocks);
         ok = ok && cudaMalloc(&D->edgeBuf, 8 * bytes) == cudaSuccess;
         ok = ok && cudaMalloc(&D->dUsed, sizeof(unsigned long long)) == cudaSuccess;
-        ok = ok && cudaMalloc(&D->dEdgeTiles, sizeof(mlp::EdgeTile) * std::max<size_t>(1, D->edgeTiles.size())) == cudaSuccess;
+        ok = ok && cudaMalloc(&D->dStepTiles, sizeof(mlp::EdgeTile) * std::max<size_t>(1, D->stepTiles.size())) == cudaSuccess;
     }
     if (D->bounded) {
         ok = ok && cudaMalloc(&D->dTiles, sizeof(TileInfo) * D->tiles.size()) == cudaSuccess;
@@ -1098,8 +1099,8 @@ int buildDomain(const std::vector<BlockSpec> &spec, const DomainOptions &o, swe_
     }
     cudaMemsetAsync(D->b, 0, bytes, D->stream);
     cudaMemcpyAsync(D->dBlocks, D->blocks.data(), sizeof(BlockDesc) * D->blocks.size(), cudaMemcpyHostToDevice, D->stream);
-    if (D->edgeBuffered && !D->edgeTiles.empty())
-        cudaMemcpyAsync(D->dEdgeTiles, D->edgeTiles.data(), sizeof(mlp::EdgeTile) * D->edgeTiles.size(),
+    if (D->edgeBuffered && !D->stepTiles.empty())
+        cudaMemcpyAsync(D->dStepTiles, D->stepTiles.data(), sizeof(mlp::EdgeTile) * D->stepTiles.size(),
                         cudaMemcpyHostToDevice, D->stream);
     cudaMemcpyAsync(D->dGroups, D->groupsInit.data(), sizeof(GroupState) * D->ngroups, cudaMemcpyHostToDevice, D->stream);
     std::vector<LtsBlock> ltsInit;
@@ -2145,13 +2146,21 @@ int swe_gpu_solve_edges(int solver, long long n, const float *hL, const float *h
 // ---------------------------------------------------------------------------
 // MLP surrogate on a domain (include/swe_gb300_mlp.h)
 // ---------------------------------------------------------------------------
+static int uploadTiles(const std::vector<mlp::EdgeTile> &tiles, mlp::EdgeTile **dev) {
+    CUDA_TRY(cudaMalloc(dev, tiles.size() * sizeof(mlp::EdgeTile)));
+    CUDA_TRY(cudaMemcpy(*dev, tiles.data(), tiles.size() * sizeof(mlp::EdgeTile), cudaMemcpyHostToDevice));
+    return SWE_GPU_OK;
+}
+/// the logger's tiles and the edge pass's, when first needed
 static int ensureEdgeTiles(swe_gpu_domain *D) {
     if (D->dEdgeTiles) return SWE_GPU_OK;
     D->edgeTiles = mlp::buildEdgeTiles(D->blocks);
-    CUDA_TRY(cudaMalloc(&D->dEdgeTiles, D->edgeTiles.size() * sizeof(mlp::EdgeTile)));
-    CUDA_TRY(cudaMemcpy(D->dEdgeTiles, D->edgeTiles.data(), D->edgeTiles.size() * sizeof(mlp::EdgeTile),
-                        cudaMemcpyHostToDevice));
-    return SWE_GPU_OK;
+    return uploadTiles(D->edgeTiles, &D->dEdgeTiles);
+}
+static int ensureStepTiles(swe_gpu_domain *D) {
+    if (D->dStepTiles) return SWE_GPU_OK;
+    D->stepTiles = mlp::buildStepTiles(D->blocks);
+    return uploadTiles(D->stepTiles, &D->dStepTiles);
 }
 
 int swe_gpu_surrogate_step(swe_gpu_domain *dom, swe_mlp *m, int nsteps, long long *surrogate_edges) {
@@ -2161,7 +2170,7 @@ int swe_gpu_surrogate_step(swe_gpu_domain *dom, swe_mlp *m, int nsteps, long lon
     if (m && mlp::deviceOf(m) != dom->device)
         return fail(SWE_GPU_ERR_INVALID, "surrogate on device %d, domain on device %d", mlp::deviceOf(m), dom->device);
     CUDA_TRY(cudaSetDevice(dom->device));
-    int rc = ensureEdgeTiles(dom);
+    int rc = ensureStepTiles(dom);
     if (rc) return rc;
     if (!dom->edgeBuf) CUDA_TRY(cudaMalloc(&dom->edgeBuf, 8 * dom->fieldElems * sizeof(float)));
     if (!dom->dUsed) CUDA_TRY(cudaMalloc(&dom->dUsed, sizeof(unsigned long long)));
@@ -2173,12 +2182,12 @@ int swe_gpu_surrogate_step(swe_gpu_domain *dom, swe_mlp *m, int nsteps, long lon
     long long maxCells = 0;
     for (const BlockDesc &B : dom->blocks) maxCells = std::max(maxCells, (long long)B.nx * B.ny);
     CUDA_TRY(cudaMemsetAsync(dom->dUsed, 0, sizeof(unsigned long long), dom->stream));
-    const int ntiles = int(dom->edgeTiles.size());
+    const int ntiles = int(dom->stepTiles.size());
     for (int i = 0; i < nsteps; i++) {
         if (i > 0 || !dom->ghostsValid) {
             if ((rc = enqueueGhost(dom, 0))) return rc;
         }
-        CUDA_TRY(mlp::launchSurrogateEdges(dom->dev, m, dom->dEdgeTiles, ntiles, u, dom->dUsed, dom->stream));
+        CUDA_TRY(mlp::launchSurrogateEdges(dom->dev, m, dom->dStepTiles, ntiles, u, dom->dUsed, dom->stream));
         CUDA_TRY(mlp::launchSurrogateDt(dom->dev, dom->ngroups, dom->stream));
         CUDA_TRY(mlp::launchSurrogateApply(dom->dev, u, int(dom->blocks.size()), maxCells, dom->stream));
         CUDA_TRY(mlp::launchSurrogateFinish(dom->dev, dom->ngroups, dom->stream));

@@ -663,7 +663,7 @@ __global__ void __launch_bounds__(128) gemmCheckKernel(int mode, const __nv_bflo
 __device__ __forceinline__ bool loadDomainEdge(const DomainDev &d, const EdgeTile &T, const BlockDesc &B, int cur, int t,
                                                float q[6], long long &oL) {
     const long long P = B.pitch;
-    oL = B.base + (long long)T.col * P + (T.j0 + t);
+    oL = B.base + (long long)T.col * P + T.j0 + (T.dir == 2 ? (long long)t * P : (long long)t);
     if (t >= T.count) return false;
     const long long oR = T.dir ? oL + 1 : oL + P;
     const float *H = pick(d.h, cur);

@@ -16,7 +16,8 @@ namespace mlp {
 /// up to 128 consecutive edges of one column of one block: x-edges
 /// (col | col+1) of rows j0 .. j0+count-1 (dir 0), or y-edges (j | j+1) of
 /// column col for j = j0 .. j0+count-1 (dir 1).  Both sides of every edge are
-/// contiguous in the column layout, so a tile's loads coalesce.
+/// contiguous in the column layout, so a tile's loads coalesce.  dir 2: the
+/// y-edges (j0 | j0+1) of columns col .. col+count-1.
 struct EdgeTile {
     int block, dir, col, j0, count;
 };
@@ -39,6 +40,25 @@ inline std::vector<EdgeTile> buildEdgeTiles(const std::vector<BlockDesc> &blocks
             for (int j0 = 1; j0 <= B.ny; j0 += 128) t.push_back({k, 0, col, j0, std::min(128, B.ny - j0 + 1)});
         for (int col = 1; col <= B.nx; col++)
             for (int j0 = 0; j0 <= B.ny; j0 += 128) t.push_back({k, 1, col, j0, std::min(128, B.ny + 1 - j0)});
+    }
+    return t;
+}
+
+/// the same edges for the edge pass.  A column has ny+1 y-edges, so where ny is
+/// a multiple of 128 its last tile would hold one edge: those blocks' lowest
+/// y-edges (0|1) go to tiles along the row instead (512-row blocks: 8 tiles per
+/// column instead of 9, the edge pass of the augmented solver at 2048^2 144 ->
+/// N us).
+inline std::vector<EdgeTile> buildStepTiles(const std::vector<BlockDesc> &blocks) {
+    std::vector<EdgeTile> t;
+    for (int k = 0; k < int(blocks.size()); k++) {
+        const BlockDesc &B = blocks[k];
+        const int first = B.ny % 128 == 0 ? 1 : 0;
+        for (int col = 0; col <= B.nx; col++)
+            for (int j0 = 1; j0 <= B.ny; j0 += 128) t.push_back({k, 0, col, j0, std::min(128, B.ny - j0 + 1)});
+        for (int col = 1; col <= B.nx; col++)
+            for (int j0 = first; j0 <= B.ny; j0 += 128) t.push_back({k, 1, col, j0, std::min(128, B.ny + 1 - j0)});
+        for (int col = 1; first && col <= B.nx; col += 128) t.push_back({k, 2, col, 0, std::min(128, B.nx + 1 - col)});
     }
     return t;
 }
