@@ -64,8 +64,14 @@ constexpr float kGateTau = 0.25f;     // |strengths - closure| <= tau (|closure|
 constexpr float kMinSpread = 0.5f;    // s2 - s1 >= 0.5 c to use the surrogate
 constexpr float kTrainSpread = 0.1f;  // s2 - s1 < 0.1 c: no gradient
 
-// forward (inference) kernel: shared memory and TMEM columns
-constexpr int kFwdX0 = kImageSmem, kFwdAct = kFwdX0 + kX0Bytes, kFwdSmem = kFwdAct + kActBytes;
+// forward (inference) kernels: kGroups groups of 128 threads, each on a tile of
+// its own, share the CTA's weights.  The features of a group's next tile use
+// its activation buffer (layer 1 has been read before its activations are
+// written), so a group needs 16 KB and 64 TMEM columns: two CTAs of four fill
+// an SM's 512 columns with 32 warps.  CTAs of one group each, with their own
+// 21 KB of weights and a feature buffer, came to 20 warps.
+constexpr int kGroups = 4;
+constexpr int kFwdAct = kImageSmem, kFwdSmem = kFwdAct + kGroups * kActBytes;
 constexpr uint32_t kFwdCols = 64;
 // training kernel: shared memory ...
 constexpr int kTrOnes = kImageSmem, kTrX0 = kTrOnes + kOnesBytes, kTrA1 = kTrX0 + kX0Bytes, kTrA2 = kTrA1 + kActBytes,
@@ -114,24 +120,46 @@ struct EdgeFeat {
     bool wet;
 };
 
-__device__ __forceinline__ void edgeFeatures(float hL, float hR, float huL, float huR, float bL, float bR, EdgeFeat &f) {
+/// the quotients and roots of edgeFeatures, with the operators of a known range
+/// (TAME) or the general ones
+template <bool TAME>
+__device__ __forceinline__ void edgeQuotients(float hL, float hR, float huL, float huR, EdgeFeat &f, float &rhm, float &rc,
+                                              float &uL, float &uR) {
     f.hm = 0.5f * (hL + hR);
-    f.c = sqrtf(kG * f.hm);
-    const float rhm = 1.f / f.hm, rc = 1.f / f.c;
-    const float uL = huL / hL, uR = huR / hR;
+    const float gh = kG * f.hm;
+    f.c = TAME ? sqrtRn(gh) : sqrtf(gh);
+    rhm = TAME ? rcpRn(f.hm) : 1.f / f.hm;
+    rc = TAME ? rcpRn(f.c) : 1.f / f.c;
+    uL = TAME ? divRn(huL, hL) : huL / hL;
+    uR = TAME ? divRn(huR, hR) : huR / hR;
+    const float sqL = TAME ? sqrtRn(hL) : sqrtf(hL), sqR = TAME ? sqrtRn(hR) : sqrtf(hR);
+    const float num = uL * sqL + uR * sqR, den = sqL + sqR;
+    // (a quotient below divRn's range is rounded away in uRoe -+ c)
+    const float uRoe = TAME ? divRn(num, den) : num / den;
+    f.s10 = uRoe - f.c;
+    f.s20 = uRoe + f.c;
+}
+/// a momentum that divRn takes: 0 or in [2^-90, 2^40]
+__device__ __forceinline__ bool tameMomentum(float m) {
+    return (fabsf(m) >= 0x1p-90f && fabsf(m) <= 0x1p40f) || m == 0.f;
+}
+
+__device__ __forceinline__ void edgeFeatures(float hL, float hR, float huL, float huR, float bL, float bR, EdgeFeat &f) {
+    float rhm, rc, uL, uR;
+    f.wet = hL >= kWet && hR >= kWet;
+    // (nothing of an edge that is not wet is used)
+    if (!f.wet || (fmaxf(hL, hR) <= 0x1p20f && tameMomentum(huL) && tameMomentum(huR)))
+        edgeQuotients<true>(hL, hR, huL, huR, f, rhm, rc, uL, uR);
+    else
+        edgeQuotients<false>(hL, hR, huL, huR, f, rhm, rc, uL, uR);
     f.x[0] = (hL - f.hm) * rhm;
     f.x[1] = (hR - f.hm) * rhm;
     f.x[2] = uL * rc;
     f.x[3] = uR * rc;
     f.x[4] = (bR - bL) * rhm;
     f.x[5] = ((hL + bL) - (hR + bR)) * rhm;
-    const float sqL = sqrtf(hL), sqR = sqrtf(hR);
-    const float uRoe = (uL * sqL + uR * sqR) / (sqL + sqR);
-    f.s10 = uRoe - f.c;
-    f.s20 = uRoe + f.c;
     f.dF1 = huR - huL;
     f.dF2 = ((huR * uR + kHalfG * hR * hR) - (huL * uL + kHalfG * hL * hL)) + kHalfG * (hL + hR) * (bR - bL);
-    f.wet = hL >= kWet && hR >= kWet;
 #pragma unroll
     for (int k = 0; k < kIn; k++) f.x[k] = f.wet ? fminf(fmaxf(f.x[k], -kClip), kClip) : 0.f;
 }
@@ -146,7 +174,7 @@ __device__ __forceinline__ void surrogateWaves(const float o[4], const EdgeFeat 
     w.s1 = fmaf(f.c, o[0], f.s10);
     w.s2 = fmaf(f.c, o[1], f.s20);
     w.D = w.s2 - w.s1;
-    const float rD = 1.f / w.D;
+    const float rD = fabsf(w.D) >= 0x1p-60f && fabsf(w.D) <= 0x1p60f ? rcpRn(w.D) : 1.f / w.D;
     w.b1 = fmaf(w.s2, f.dF1, -f.dF2) * rD;
     w.b2 = fmaf(-w.s1, f.dF1, f.dF2) * rD;
     const float hc = f.hm * f.c;
@@ -238,7 +266,7 @@ __device__ __forceinline__ void epilogueSilu(uint32_t tz, const float *hbias, ui
 }
 /// backward epilogue: dZ = bf16(dA * silu'(Z + b)) for this thread's row
 __device__ __forceinline__ void epilogueDsilu(uint32_t tda, uint32_t tz, const float *bias, uint8_t *dst, int row) {
-#pragma unroll
+#pragma unroll 1
     for (int c = 0; c < kHid; c += 16) {
         float g[16], z[16];
         tc::load16(tda, c, g);
@@ -251,17 +279,31 @@ __device__ __forceinline__ void epilogueDsilu(uint32_t tda, uint32_t tz, const f
     }
 }
 
-/// all threads: make this thread's shared-memory writes and TMEM reads
-/// ordered before MMAs that one thread issues after the barrier
-__device__ __forceinline__ void publishToMma() {
+/// barrier of one 128-thread group of the CTA (named barrier 1 + group)
+__device__ __forceinline__ void groupSync(int group) { asm volatile("bar.sync %0, 128;" ::"r"(group + 1) : "memory"); }
+/// whether `v` holds in every thread of the group
+__device__ __forceinline__ bool groupAll(int group, bool v) {
+    uint32_t r;
+    asm volatile("{\n.reg .pred p, q;\nsetp.ne.b32 p, %2, 0;\nbarrier.cta.red.and.pred q, %1, 128, p;\nselp.u32 %0, 1, 0, q;\n}"
+                 : "=r"(r)
+                 : "r"(group + 1), "r"(v ? 1 : 0)
+                 : "memory");
+    return r != 0;
+}
+
+/// every thread of the group: make this thread's shared-memory writes and TMEM
+/// reads ordered before MMAs that one thread issues after the barrier
+__device__ __forceinline__ void publishToMma(int group) {
     tc::fenceSmemForMma();
     tc::fenceBeforeSync();
-    __syncthreads();
+    groupSync(group);
     tc::fenceAfterSync();
 }
-/// all threads: wait for the committed MMAs; false (everywhere) on time-out
+/// wait for the committed MMAs; false on time-out.  A thread that timed out
+/// goes on with its tile (the group leaves together, by groupAll at its end).
 __device__ __forceinline__ bool awaitMma(uint64_t *mbar, uint32_t &phase) {
-    const bool ok = __syncthreads_and(tc::mbarWait(mbar, phase));
+    const bool ok = tc::mbarWait(mbar, phase);
+    __syncwarp();
     phase ^= 1u;
     tc::fenceAfterSync();
     return ok;
@@ -278,43 +320,92 @@ __device__ __forceinline__ void stageImage(const uint8_t *image, uint8_t *s, flo
 }
 
 /// the four forward GEMMs of one tile, with the epilogues between them; on
-/// return the raw outputs sit in TMEM columns oCol.. (without b4).  act[l] is
-/// the shared-memory buffer of layer l's output activations, zc[l] the TMEM
-/// columns of its pre-activations.
-__device__ __forceinline__ bool forwardTile(uint32_t tm, const uint8_t *sW, const float *hbias, const uint8_t *sX0,
-                                            uint8_t *const act[3], const uint32_t zc[3], uint32_t oCol, uint64_t *mbar,
-                                            uint32_t &phase) {
-    const int t = threadIdx.x;
-    publishToMma();
-    if (t == 0) {
-        tc::mma(tm + zc[0], tc::smemDesc(sX0, 0, kInPad), tc::smemDesc(sW + pW1, 0, kInPad), tc::idescBf16(128, kHid), false);
-        tc::commit(mbar);
-    }
-    if (!awaitMma(mbar, phase)) return false;
-    epilogueSilu(tm + zc[0], hbias, act[0], t);
-    const int pw[2] = {pW2, pW3};
-#pragma unroll
-    for (int l = 0; l < 2; l++) {
-        publishToMma();
+/// return the raw outputs sit in TMEM columns oCol.. (without b4).  Layer l's
+/// activations go to act + l actStride, its pre-activations to TMEM columns
+/// l zStride; t is the thread's number in its group.  The layers share one copy
+/// of the code: unrolled, the training kernel's single pass over it waited for
+/// instructions more than for anything else.
+__device__ __forceinline__ bool forwardTile(int group, int t, uint32_t tm, const uint8_t *sW, const float *hbias,
+                                            const uint8_t *sX0, uint8_t *act, int actStride, uint32_t zStride, uint32_t oCol,
+                                            uint64_t *mbar, uint32_t &phase) {
+    bool ok = true;
+#pragma unroll 1
+    for (int l = 0; l < 3; l++) {
+        publishToMma(group);
+        uint8_t *const a = act + l * actStride;
+        const uint32_t z = tm + l * zStride;
         if (t == 0) {
+            if (l == 0) {
+                tc::mma(z, tc::smemDesc(sX0, 0, kInPad), tc::smemDesc(sW + pW1, 0, kInPad), tc::idescBf16(128, kHid), false);
+            } else {
+                const uint8_t *in = a - actStride, *wl = sW + pW2 + (l - 1) * (pW3 - pW2);
 #pragma unroll
-            for (int kk = 0; kk < kHid / 16; kk++)
-                tc::mma(tm + zc[l + 1], tc::smemDesc(act[l], kk * 16, kHid), tc::smemDesc(sW + pw[l], kk * 16, kHid),
-                        tc::idescBf16(128, kHid), kk > 0);
+                for (int kk = 0; kk < kHid / 16; kk++)
+                    tc::mma(z, tc::smemDesc(in, kk * 16, kHid), tc::smemDesc(wl, kk * 16, kHid), tc::idescBf16(128, kHid),
+                            kk > 0);
+            }
             tc::commit(mbar);
         }
-        if (!awaitMma(mbar, phase)) return false;
-        epilogueSilu(tm + zc[l + 1], hbias + kHid * (l + 1), act[l + 1], t);
+        __syncwarp();
+        ok = awaitMma(mbar, phase) && ok;
+        epilogueSilu(z, hbias + kHid * l, a, t);
     }
-    publishToMma();
+    publishToMma(group);
     if (t == 0) {
 #pragma unroll
         for (int kk = 0; kk < kHid / 16; kk++)
-            tc::mma(tm + oCol, tc::smemDesc(act[2], kk * 16, kHid), tc::smemDesc(sW + pW4, kk * 16, kHid),
+            tc::mma(tm + oCol, tc::smemDesc(act + 2 * actStride, kk * 16, kHid), tc::smemDesc(sW + pW4, kk * 16, kHid),
                     tc::idescBf16(128, kOutPad), kk > 0);
         tc::commit(mbar);
     }
-    return awaitMma(mbar, phase);
+    __syncwarp();
+    return awaitMma(mbar, phase) && ok;
+}
+
+/// What a group of the forward kernels works with
+struct FwdGroup {
+    int id, t;           // group of the CTA, thread of the group
+    uint32_t tm;         // its TMEM columns
+    uint8_t *act;        // its activation (and feature) buffer
+    const uint8_t *sW;
+    const float *hbias, *bias;
+    uint64_t *mbar;
+    uint32_t phase;
+};
+/// a forward CTA's set-up: weights, TMEM columns, a barrier per group
+__device__ __forceinline__ FwdGroup fwdBegin(const uint8_t *image, uint8_t *smem, uint64_t *mbar, uint32_t *tslot, float *sHb) {
+    stageImage(image, smem, sHb);
+    if (threadIdx.x == 0)
+        for (int g = 0; g < kGroups; g++) tc::mbarInit(mbar + g, 1);
+    if (threadIdx.x < 32) tc::tmemAlloc(tslot, kFwdCols * kGroups);
+    tc::fenceSmemForMma();
+    tc::fenceBeforeSync();
+    __syncthreads();
+    tc::fenceAfterSync();
+    const int id = int(threadIdx.x >> 7);
+    return FwdGroup{id, int(threadIdx.x & 127), *tslot + kFwdCols * id, smem + kFwdAct + id * kActBytes, smem, sHb,
+                    reinterpret_cast<const float *>(smem + pBias), mbar + id, 0u};
+}
+/// network outputs of the group's tile (features x); false on time-out
+__device__ __forceinline__ bool fwdTile(FwdGroup &G, const float x[kIn], float o[4]) {
+    storeX0(G.act, G.t, x);
+    const bool ok = forwardTile(G.id, G.t, G.tm, G.sW, G.hbias, G.act, G.act, 0, 0, 0, G.mbar, G.phase);
+    float v[16];
+    tc::load16(G.tm, 0, v);
+#pragma unroll
+    for (int k = 0; k < 4; k++) o[k] = v[k] + G.bias[3 * kHid + k];
+    return ok;
+}
+/// leaves the CTA's TMEM; a group that timed out waits (bounded) for an MMA
+/// still in flight before the columns go
+__device__ __forceinline__ void fwdEnd(FwdGroup &G, bool ok, uint32_t tslot, int *err) {
+    if (!ok) {
+        if (G.t == 0) atomicOr(err, 1);
+        tc::mbarWait(G.mbar, G.phase);
+    }
+    tc::fenceBeforeSync();
+    __syncthreads();
+    if (threadIdx.x < 32) tc::tmemFree(tslot, kFwdCols * kGroups);
 }
 
 /// edges in structure-of-arrays form: quantity k of edge e at v[k * stride + idx(e)]
@@ -332,47 +423,29 @@ enum FwdMode { FWD_OUTPUTS = 0, FWD_SOLVE = 1 };
 /// inference: outputs (FWD_OUTPUTS: raw network outputs o, 4 x n) or the
 /// surrogate solve (FWD_SOLVE: net updates 4 x n, speed, used flag per edge)
 template <int MODE>
-__global__ void __launch_bounds__(128) forwardKernel(const uint8_t *image, EdgeBatch in, float *out, float *speed,
-                                                     uint8_t *used, long long ostride, int *err) {
+__global__ void __launch_bounds__(128 * kGroups, 2) forwardKernel(const uint8_t *image, EdgeBatch in, float *out, float *speed,
+                                                                  uint8_t *used, long long ostride, int *err) {
     extern __shared__ __align__(1024) uint8_t smem[];
-    __shared__ __align__(8) uint64_t mbar;
+    __shared__ __align__(8) uint64_t mbar[kGroups];
     __shared__ uint32_t tslot;
-    __shared__ float sHb[3 * kHid];  // halved hidden-layer biases
-    const int t = threadIdx.x;
-    uint8_t *sW = smem, *sX0 = smem + kFwdX0, *sAct = smem + kFwdAct;
-    stageImage(image, sW, sHb);
-    if (t == 0) tc::mbarInit(&mbar, 1);
-    if (t < 32) tc::tmemAlloc(&tslot, kFwdCols);
-    tc::fenceBeforeSync();
-    __syncthreads();
-    tc::fenceAfterSync();
-    const uint32_t tm = tslot;
-    const float *bias = reinterpret_cast<const float *>(sW + pBias);
-    uint8_t *const act[3] = {sAct, sAct, sAct};
-    const uint32_t zc[3] = {0, 0, 0};
-    uint32_t phase = 0;
+    __shared__ __align__(16) float sHb[3 * kHid];  // halved hidden-layer biases
+    FwdGroup G = fwdBegin(image, smem, mbar, &tslot, sHb);
     bool ok = true;
     const int ntiles = (in.count + kTile - 1) / kTile;
-    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const int i = tile * kTile + t;
+    for (int tile = blockIdx.x * kGroups + G.id; ok && tile < ntiles; tile += gridDim.x * kGroups) {
+        const int i = tile * kTile + G.t;
         const bool valid = i < in.count;
         float q[6] = {1.f, 1.f, 0.f, 0.f, 0.f, 0.f};
-        long long e = 0;
         if (valid) {
-            e = in.index(i);
+            const long long e = in.index(i);
 #pragma unroll
             for (int k = 0; k < 6; k++) q[k] = __ldg(in.v + k * in.stride + e);
         }
         EdgeFeat f;
         edgeFeatures(q[0], q[1], q[2], q[3], q[4], q[5], f);
-        storeX0(sX0, t, f.x);
-        if (!(ok = forwardTile(tm, sW, sHb, sX0, act, zc, 0, &mbar, phase))) break;
-        float v[16];
-        tc::load16(tm, 0, v);
         float o[4];
-#pragma unroll
-        for (int k = 0; k < 4; k++) o[k] = v[k] + bias[3 * kHid + k];
-        if (!valid) continue;
+        ok = fwdTile(G, f.x, o);
+        if (!(ok = groupAll(G.id, ok)) || !valid) continue;
         if (MODE == FWD_OUTPUTS) {
 #pragma unroll
             for (int k = 0; k < 4; k++) out[k * ostride + i] = o[k];
@@ -394,13 +467,7 @@ __global__ void __launch_bounds__(128) forwardKernel(const uint8_t *image, EdgeB
             used[i] = use ? 1 : 0;
         }
     }
-    if (!ok) {
-        if (t == 0) atomicOr(err, 1);
-        tc::mbarWait(&mbar, phase);  // bounded: let an MMA still in flight finish before the columns go
-    }
-    tc::fenceBeforeSync();
-    __syncthreads();
-    if (t < 32) tc::tmemFree(tm, kFwdCols);
+    fwdEnd(G, ok, tslot, err);
 }
 
 /// training: forward, loss and backward over the batch's tiles; each CTA
@@ -411,11 +478,11 @@ __global__ void __launch_bounds__(128, 1) trainKernel(const uint8_t *image, Edge
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ __align__(8) uint64_t mbar;
     __shared__ uint32_t tslot;
-    __shared__ float sHb[3 * kHid];  // halved hidden-layer biases
+    __shared__ __align__(16) float sHb[3 * kHid];  // halved hidden-layer biases
     __shared__ float warpLoss[4];
     const int t = threadIdx.x;
     uint8_t *sW = smem, *sOnes = smem + kTrOnes, *sX0 = smem + kTrX0, *sDZ4 = smem + kTrDZ4, *sDZ = smem + kTrDZ;
-    uint8_t *const act[3] = {smem + kTrA1, smem + kTrA2, smem + kTrA3};
+    uint8_t *const act = smem + kTrA1;  // A1, A2, A3
     stageImage(image, sW, sHb);
     for (int i = t; i < kOnesBytes / 4; i += blockDim.x) reinterpret_cast<uint32_t *>(sOnes)[i] = 0x3F803F80u;  // BF16 1.0
     for (int i = t; i < (kTrEnd - kTrDZ4) / 4; i += blockDim.x) reinterpret_cast<uint32_t *>(sDZ4)[i] = 0u;
@@ -426,7 +493,6 @@ __global__ void __launch_bounds__(128, 1) trainKernel(const uint8_t *image, Edge
     tc::fenceAfterSync();
     const uint32_t tm = tslot;
     const float *bias = reinterpret_cast<const float *>(sW + pBias);
-    const uint32_t zc[3] = {cZ1, cZ2, cZ3};
     uint32_t phase = 0;
     bool ok = true, first = true;
     float lossSum = 0.f;
@@ -445,7 +511,7 @@ __global__ void __launch_bounds__(128, 1) trainKernel(const uint8_t *image, Edge
         EdgeFeat f;
         edgeFeatures(q[0], q[1], q[2], q[3], q[4], q[5], f);
         storeX0(sX0, t, f.x);
-        if (!(ok = forwardTile(tm, sW, sHb, sX0, act, zc, cO, &mbar, phase))) break;
+        ok = forwardTile(0, t, tm, sW, sHb, sX0, act, kActBytes, cZ2 - cZ1, cO, &mbar, phase);
         // loss and dLoss/dO
         {
             float v[16];
@@ -457,50 +523,52 @@ __global__ void __launch_bounds__(128, 1) trainKernel(const uint8_t *image, Edge
             storeDZ4(sDZ4, t, dO);
         }
         // layer 4: dA3 = dZ4 W4; gW4^T += A3^T dZ4; db4 += dZ4^T 1
-        publishToMma();
+        publishToMma(0);
         if (t == 0) {
             tc::mma(tm + cDA, tc::smemDesc(sDZ4, 0, kOutPad), tc::smemDescMN(sW + pW4, 0, kHid),
                     tc::idescBf16(128, kHid, false, true), false);
-#pragma unroll
+#pragma unroll 2
             for (int kk = 0; kk < kTile / 16; kk++) {
                 const bool acc = !(first && kk == 0);
-                tc::mma(tm + cGW4, tc::smemDescMN(act[2], kk * 16, kHid), tc::smemDescMN(sDZ4, kk * 16, kOutPad),
+                tc::mma(tm + cGW4, tc::smemDescMN(act + 2 * kActBytes, kk * 16, kHid), tc::smemDescMN(sDZ4, kk * 16, kOutPad),
                         tc::idescBf16(128, kOutPad, true, true), acc);
                 tc::mma(tm + cDB4, tc::smemDescMN(sDZ4, kk * 16, kOutPad), tc::smemDesc(sOnes, kk * 16, kTile),
                         tc::idescBf16(128, 16, true, false), acc);
             }
             tc::commit(&mbar);
         }
-        if (!(ok = awaitMma(&mbar, phase))) break;
+        __syncwarp();
+        ok = awaitMma(&mbar, phase) && ok;
         // layers 3, 2, 1: dZ_l = dA_l * silu'(Z_l); dA_{l-1} = dZ_l W_l; gW_l += dZ_l^T A_{l-1}; db_l += dZ_l^T 1
-        const int pw[3] = {pW1, pW2, pW3};
-        const uint32_t cgw[3] = {cGW1, cGW2, cGW3}, cdb[3] = {cDB1, cDB2, cDB3};
-#pragma unroll
+#pragma unroll 1
         for (int l = 2; l >= 0; l--) {
-            epilogueDsilu(tm + cDA, tm + zc[l], bias + kHid * l, sDZ, t);
-            publishToMma();
+            epilogueDsilu(tm + cDA, tm + cZ1 + l * (cZ2 - cZ1), bias + kHid * l, sDZ, t);
+            publishToMma(0);
             if (t == 0) {
                 if (l > 0) {
+                    const uint8_t *wl = sW + pW2 + (l - 1) * (pW3 - pW2);
 #pragma unroll
                     for (int kk = 0; kk < kHid / 16; kk++)
-                        tc::mma(tm + cDA, tc::smemDesc(sDZ, kk * 16, kHid), tc::smemDescMN(sW + pw[l], kk * 16, kHid),
+                        tc::mma(tm + cDA, tc::smemDesc(sDZ, kk * 16, kHid), tc::smemDescMN(wl, kk * 16, kHid),
                                 tc::idescBf16(128, kHid, false, true), kk > 0);
                 }
-                const uint8_t *prev = l > 0 ? act[l - 1] : sX0;
+                const uint8_t *prev = l > 0 ? act + (l - 1) * kActBytes : sX0;
                 const int pwid = l > 0 ? kHid : kInPad;
-#pragma unroll
+                const uint32_t gw = tm + (l == 2 ? cGW3 : l == 1 ? cGW2 : cGW1), db = tm + (l == 2 ? cDB3 : l == 1 ? cDB2 : cDB1);
+#pragma unroll 2
                 for (int kk = 0; kk < kTile / 16; kk++) {
                     const bool acc = !(first && kk == 0);
-                    tc::mma(tm + cgw[l], tc::smemDescMN(sDZ, kk * 16, kHid), tc::smemDescMN(prev, kk * 16, pwid),
+                    tc::mma(gw, tc::smemDescMN(sDZ, kk * 16, kHid), tc::smemDescMN(prev, kk * 16, pwid),
                             tc::idescBf16(128, pwid, true, true), acc);
-                    tc::mma(tm + cdb[l], tc::smemDescMN(sDZ, kk * 16, kHid), tc::smemDesc(sOnes, kk * 16, kTile),
+                    tc::mma(db, tc::smemDescMN(sDZ, kk * 16, kHid), tc::smemDesc(sOnes, kk * 16, kTile),
                             tc::idescBf16(128, 16, true, false), acc);
                 }
                 tc::commit(&mbar);
             }
-            if (!(ok = awaitMma(&mbar, phase))) break;
+            __syncwarp();
+            ok = awaitMma(&mbar, phase) && ok;
         }
-        if (!ok) break;
+        if (!(ok = groupAll(0, ok))) break;
         first = false;
     }
     // per-CTA partial gradients: rows 0..63 of the accumulators live in the lanes of warps 0 and 1
@@ -512,13 +580,13 @@ __global__ void __launch_bounds__(128, 1) trainKernel(const uint8_t *image, Edge
         }
         if (!first) tc::load16(tm + cGW1, 0, v);
         for (int k = 0; k < kIn; k++) P[oW1 + t * kIn + k] = v[k];
-        for (int l = 0; l < 2; l++) {
-            const uint32_t col = l == 0 ? cGW2 : cGW3;
-            const int off = l == 0 ? oW2 : oW3;
-            for (int c = 0; c < kHid; c += 16) {
-                if (!first) tc::load16(tm + col, c, v);
-                for (int k = 0; k < 16; k++) P[off + t * kHid + c + k] = v[k];
-            }
+        static_assert(oW2 % 4 == 0 && oW3 % 4 == 0 && kPartStride % 4 == 0, "16-byte stores");
+#pragma unroll 1
+        for (int q = 0; q < 2 * kHid; q += 16) {
+            if (!first) tc::load16(tm + cGW2, q, v);  // gW2, then gW3 behind it
+            float4 *dst = reinterpret_cast<float4 *>(P + (q < kHid ? oW2 + t * kHid + q : oW3 + t * kHid + q - kHid));
+#pragma unroll
+            for (int k = 0; k < 4; k++) dst[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
         }
         if (!first) tc::load16(tm + cGW4, 0, v);
         for (int k = 0; k < kOut; k++) P[oW4 + k * kHid + t] = v[k];
@@ -543,25 +611,62 @@ __global__ void __launch_bounds__(128, 1) trainKernel(const uint8_t *image, Edge
     if (t < 32) tc::tmemFree(tm, kTrCols);
 }
 
+/// where the packed image holds parameter i: the byte offset of its BF16 weight,
+/// or of its FP32 bias with the sign bit set
+__device__ __forceinline__ int imageOffset(int i) {
+    if (i < oB1) return pW1 + int(tc::coreOffset(i / kIn, i % kIn, kInPad));
+    if (i < oW2) return ~(pBias + 4 * (i - oB1));
+    if (i < oB2) return pW2 + int(tc::coreOffset((i - oW2) / kHid, (i - oW2) % kHid, kHid));
+    if (i < oW3) return ~(pBias + 4 * (kHid + i - oB2));
+    if (i < oB3) return pW3 + int(tc::coreOffset((i - oW3) / kHid, (i - oW3) % kHid, kHid));
+    if (i < oW4) return ~(pBias + 4 * (2 * kHid + i - oB3));
+    if (i < oB4) return pW4 + int(tc::coreOffset((i - oW4) / kHid, (i - oW4) % kHid, kHid));
+    return ~(pBias + 4 * (3 * kHid + i - oB4));
+}
+
 /// sum of the per-CTA partials (fixed order); optional Adam step (Kingma & Ba
-/// 2015) on the FP32 master parameters
-__global__ void reduceAdamKernel(const float *partials, int nparts, float *grad, float *lossOut, float *p, float *m,
-                                 float *v, float lr, float beta1, float beta2, float eps, float bc1, float bc2) {
+/// 2015) on the FP32 master parameters, written to the packed image too (its
+/// padding stays as packKernel left it).  Latency alone: the partials are loaded
+/// 16 at a time, and small CTAs spread the parameters over the SMs.
+__global__ void __launch_bounds__(64) reduceAdamKernel(const float *partials, int nparts, float *grad, float *lossOut, float *p,
+                                                       float *m, float *v, float lr, float beta1, float beta2, float eps,
+                                                       float bc1, float bc2, uint8_t *image) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i > kNParams) return;
+    float mi = 0.f, vi = 0.f, pi = 0.f;
+    const bool adam = lr > 0.f && i < kNParams;
+    if (adam) {
+        mi = m[i];
+        vi = v[i];
+        pi = p[i];
+    }
     float g = 0.f;
-    for (int c = 0; c < nparts; c++) g += partials[(long long)c * kPartStride + i];
+    int c = 0;
+    for (; c + 16 <= nparts; c += 16) {
+        float x[16];
+#pragma unroll
+        for (int k = 0; k < 16; k++) x[k] = partials[(long long)(c + k) * kPartStride + i];
+#pragma unroll
+        for (int k = 0; k < 16; k++) g += x[k];
+    }
+    for (; c < nparts; c++) g += partials[(long long)c * kPartStride + i];
     if (i == kNParams) {
         if (lossOut) *lossOut = g;
         return;
     }
     if (grad) grad[i] = g;
-    if (lr > 0.f) {
-        const float mi = fmaf(beta1, m[i], (1.f - beta1) * g);
-        const float vi = fmaf(beta2, v[i], (1.f - beta2) * g * g);
+    if (adam) {
+        mi = fmaf(beta1, mi, (1.f - beta1) * g);
+        vi = fmaf(beta2, vi, (1.f - beta2) * g * g);
         m[i] = mi;
         v[i] = vi;
-        p[i] -= lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
+        pi -= lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
+        p[i] = pi;
+        const int o = imageOffset(i);
+        if (o >= 0)
+            *reinterpret_cast<__nv_bfloat16 *>(image + o) = __float2bfloat16_rn(pi);
+        else
+            *reinterpret_cast<float *>(image + ~o) = pi;
     }
 }
 
@@ -677,89 +782,64 @@ __device__ __forceinline__ bool loadDomainEdge(const DomainDev &d, const EdgeTil
     return true;
 }
 
-/// the CTA's running max wave speed goes to its group
-__device__ __forceinline__ void flushSpeed(const DomainDev &d, int group, float &smax, float *sMax) {
+/// the warp's running max wave speed goes to its group
+__device__ __forceinline__ void flushSpeed(const DomainDev &d, int group, float &smax) {
     float v = smax;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v = vmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-    if ((threadIdx.x & 31) == 0) sMax[threadIdx.x >> 5] = v;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const float m = vmax(vmax(sMax[0], sMax[1]), vmax(sMax[2], sMax[3]));
-        atomicMax(&d.groups[group].speedBits, __float_as_uint(m));
-    }
-    __syncthreads();
+    if ((threadIdx.x & 31) == 0) atomicMax(&d.groups[group].speedBits, __float_as_uint(v));
     smax = 0.f;
 }
 
-/// edge pass over a contiguous range of tiles per CTA (so the group changes
-/// rarely within a CTA).  SURR: surrogate with the gate, else the augmented
-/// solver on every edge (the default step of augmented-solver domains).
-/// Groups whose time reached their target (or that sit the step out) are
-/// skipped, in this and the following kernels of the step.
-template <bool SURR>
-__global__ void __launch_bounds__(128) surrogateEdgeKernel(const DomainDev d, const uint8_t *image, const EdgeTile *tiles,
-                                                           int ntiles, EdgeUpdates u, unsigned long long *usedCount,
-                                                           int *err) {
+/// Edge pass over a contiguous range of tiles per group of 128 threads (so the
+/// dt group changes rarely): the surrogate with the gate.  Groups whose time
+/// reached their target (or that sit the step out) are skipped, in this and
+/// the following kernels of the step.
+///
+/// Bound by the special-function unit: 192 tanh and some 10 roots and quotients
+/// an edge are 370 us for the 8.4 M edges of 2048^2.  650 us as CTAs of one group
+/// (20 warps per SM), 570 us now (32 warps).
+__global__ void __launch_bounds__(128 * kGroups, 2)
+    surrogateEdgeKernel(const DomainDev d, const uint8_t *image, const EdgeTile *tiles, int ntiles, EdgeUpdates u,
+                        unsigned long long *usedCount, int *err) {
     extern __shared__ __align__(1024) uint8_t smem[];
-    __shared__ __align__(8) uint64_t mbar;
+    __shared__ __align__(8) uint64_t mbar[kGroups];
     __shared__ uint32_t tslot;
-    __shared__ float sHb[3 * kHid];  // halved hidden-layer biases
-    __shared__ float sMax[4];
-    const int t = threadIdx.x;
-    uint8_t *sW = smem, *sX0 = smem + kFwdX0, *sAct = smem + kFwdAct;
-    uint32_t tm = 0;
-    if (SURR) {
-        stageImage(image, sW, sHb);
-        if (t == 0) tc::mbarInit(&mbar, 1);
-        if (t < 32) tc::tmemAlloc(&tslot, kFwdCols);
-        tc::fenceBeforeSync();
-        __syncthreads();
-        tc::fenceAfterSync();
-        tm = tslot;
-    }
-    const float *bias = reinterpret_cast<const float *>(sW + pBias);
-    uint8_t *const act[3] = {sAct, sAct, sAct};
-    const uint32_t zc[3] = {0, 0, 0};
-    uint32_t phase = 0;
+    __shared__ __align__(16) float sHb[3 * kHid];  // halved hidden-layer biases
+    FwdGroup G = fwdBegin(image, smem, mbar, &tslot, sHb);
+    const int t = G.t;
     bool ok = true;
     float smax = 0.f;
     unsigned usedLocal = 0;
-    const int first = int((long long)ntiles * blockIdx.x / gridDim.x);
-    const int last = int((long long)ntiles * (blockIdx.x + 1) / gridDim.x);
+    const int worker = blockIdx.x * kGroups + G.id, workers = gridDim.x * kGroups;
+    const int first = int((long long)ntiles * worker / workers);
+    const int last = int((long long)ntiles * (worker + 1) / workers);
     int group = -1;
-    for (int tile = first; tile < last; tile++) {
+    for (int tile = first; ok && tile < last; tile++) {
         const EdgeTile T = tiles[tile];
         const BlockDesc &B = d.blocks[T.block];
         if (B.group != group) {
-            if (group >= 0) flushSpeed(d, group, smax, sMax);
+            if (group >= 0) flushSpeed(d, group, smax);
             group = B.group;
         }
-        if (!groupActive(d.groups + group)) continue;  // the group reached its target (CTA-uniform)
+        if (!groupActive(d.groups + group)) continue;  // the dt group reached its target (uniform)
         const int cur = d.groups[group].cur;
         float q[6] = {1.f, 1.f, 0.f, 0.f, 0.f, 0.f};
         long long oL;
         const bool valid = loadDomainEdge(d, T, B, cur, t, q, oL);
         float upd[4], s = 0.f;
-        bool use = false;
-        if (SURR) {
-            EdgeFeat f;
-            edgeFeatures(q[0], q[1], q[2], q[3], q[4], q[5], f);
-            storeX0(sX0, t, f.x);
-            if (!(ok = forwardTile(tm, sW, sHb, sX0, act, zc, 0, &mbar, phase))) break;
-            float v[16];
-            tc::load16(tm, 0, v);
-            float o[4];
+        EdgeFeat f;
+        edgeFeatures(q[0], q[1], q[2], q[3], q[4], q[5], f);
+        float o[4];
+        ok = fwdTile(G, f.x, o);
+        if (!(ok = groupAll(G.id, ok))) break;
+        Waves w;
+        surrogateWaves(o, f, w);
+        const bool use = valid && surrogateGate(f, w);
+        if (use) {
 #pragma unroll
-            for (int k = 0; k < 4; k++) o[k] = v[k] + bias[3 * kHid + k];
-            Waves w;
-            surrogateWaves(o, f, w);
-            use = valid && surrogateGate(f, w);
-            if (use) {
-#pragma unroll
-                for (int k = 0; k < 4; k++) upd[k] = w.U[k];
-                s = fmaxf(fabsf(w.s1), fabsf(w.s2));
-            }
+            for (int k = 0; k < 4; k++) upd[k] = w.U[k];
+            s = fmaxf(fabsf(w.s1), fabsf(w.s2));
         }
         if (valid) {
             if (!use) edgeAugRie(q[0], q[1], q[2], q[3], q[4], q[5], upd[0], upd[1], upd[2], upd[3], s);
@@ -770,19 +850,44 @@ __global__ void __launch_bounds__(128) surrogateEdgeKernel(const DomainDev d, co
             usedLocal += use ? 1u : 0u;
         }
     }
-    if (ok && group >= 0) flushSpeed(d, group, smax, sMax);
+    __syncwarp();
+    if (ok && group >= 0) flushSpeed(d, group, smax);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) usedLocal += __shfl_xor_sync(0xffffffffu, usedLocal, o);
     if ((t & 31) == 0 && usedLocal) atomicAdd(usedCount, (unsigned long long)usedLocal);
-    if (SURR) {
-        if (!ok) {
-            if (t == 0) atomicOr(err, 1);
-            tc::mbarWait(&mbar, phase);  // bounded
+    fwdEnd(G, ok, tslot, err);
+}
+
+/// the same pass with the augmented solver on every edge (the default step of
+/// augmented-solver domains)
+__global__ void __launch_bounds__(128, 12) augEdgeKernel(const DomainDev d, const EdgeTile *tiles, int ntiles, EdgeUpdates u) {
+    const int t = threadIdx.x;
+    float smax = 0.f;
+    const int first = int((long long)ntiles * blockIdx.x / gridDim.x);
+    const int last = int((long long)ntiles * (blockIdx.x + 1) / gridDim.x);
+    int group = -1;
+    for (int tile = first; tile < last; tile++) {
+        const EdgeTile T = tiles[tile];
+        const BlockDesc &B = d.blocks[T.block];
+        if (B.group != group) {
+            if (group >= 0) flushSpeed(d, group, smax);
+            group = B.group;
         }
-        tc::fenceBeforeSync();
-        __syncthreads();
-        if (t < 32) tc::tmemFree(tm, kFwdCols);
+        if (!groupActive(d.groups + group)) continue;
+        const int cur = d.groups[group].cur;
+        float q[6] = {1.f, 1.f, 0.f, 0.f, 0.f, 0.f};
+        long long oL;
+        const bool valid = loadDomainEdge(d, T, B, cur, t, q, oL);
+        float upd[4], s = 0.f;
+        if (valid) {
+            edgeAugRie(q[0], q[1], q[2], q[3], q[4], q[5], upd[0], upd[1], upd[2], upd[3], s);
+            float *const *dst = T.dir ? u.y : u.x;
+#pragma unroll
+            for (int k = 0; k < 4; k++) dst[k][oL] = upd[k];
+            smax = vmax(smax, s);
+        }
     }
+    if (group >= 0) flushSpeed(d, group, smax);
 }
 
 /// maxTimestep of every group from the edge pass's max wave speed
@@ -965,10 +1070,9 @@ struct swe_mlp {
             bc1 = 1.f - std::pow(0.9f, float(adamSteps));
             bc2 = 1.f - std::pow(0.999f, float(adamSteps));
         }
-        reduceAdamKernel<<<(kNParams + 1 + 255) / 256, 256>>>(partials, grid, gradDst, lossDst, p, m, v, lr, 0.9f, 0.999f,
-                                                               1e-8f, bc1, bc2);
+        reduceAdamKernel<<<(kNParams + 1 + 63) / 64, 64>>>(partials, grid, gradDst, lossDst, p, m, v, lr, 0.9f, 0.999f, 1e-8f,
+                                                           bc1, bc2, image);
         MLP_TRY(cudaGetLastError());
-        if (lr > 0.f) return pack();
         return SWE_GPU_OK;
     }
 };
@@ -1030,23 +1134,24 @@ int swe_mlp_create(unsigned long long seed, swe_mlp **out) {
     smemAttr((const void *)trainKernel, kTrSmem);
     smemAttr((const void *)forwardKernel<FWD_OUTPUTS>, kFwdSmem);
     smemAttr((const void *)forwardKernel<FWD_SOLVE>, kFwdSmem);
-    smemAttr((const void *)surrogateEdgeKernel<true>, kFwdSmem);
+    smemAttr((const void *)surrogateEdgeKernel, kFwdSmem);
     // resident inference CTAs per SM from their shared-memory footprint (the
     // CTA's static and dynamic shared memory plus the 1 KB the SM reserves per
-    // CTA) and registers; TMEM: every resident CTA holds kFwdCols of the SM's
-    // 512 columns.  Extra CTAs of a grid only queue.
+    // CTA) and registers; TMEM: every resident CTA holds kFwdCols x kGroups of
+    // the SM's 512 columns.  Extra CTAs of a grid only queue.  (The runtime's
+    // occupancy calculator answers 1 for any kernel that allocates TMEM.)
     int smemSm = 0, regsSm = 0;
     cudaFuncAttributes fa{}, ea{};
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&smemSm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, m->device);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&regsSm, cudaDevAttrMaxRegistersPerMultiprocessor, m->device);
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, forwardKernel<FWD_SOLVE>);
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&ea, surrogateEdgeKernel<true>);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&ea, surrogateEdgeKernel);
     if (e != cudaSuccess) return bail(mlpFail(SWE_GPU_ERR_CUDA, "create: %s", cudaGetErrorString(e)));
     const int staticSmem = int(std::max(fa.sharedSizeBytes, ea.sharedSizeBytes));
     const int regs = std::max(fa.numRegs, ea.numRegs);
     const int bySmem = smemSm / (kFwdSmem + staticSmem + 1024);
-    const int byRegs = regs > 0 ? regsSm / (regs * 128) : 8;
-    m->fwdBlocksPerSm = std::max(1, std::min(std::min(bySmem, byRegs), int(512 / kFwdCols)));
+    const int byRegs = regs > 0 ? regsSm / (regs * 128 * kGroups) : 2;
+    m->fwdBlocksPerSm = std::max(1, std::min(std::min(bySmem, byRegs), int(512 / (kFwdCols * kGroups))));
     const size_t pb = kNParams * sizeof(float);
     e = cudaMalloc(&m->p, pb);
     if (e == cudaSuccess) e = cudaMalloc(&m->m, pb);
@@ -1105,8 +1210,8 @@ int swe_mlp_forward(swe_mlp *m, int n, const float *edges, float *out) {
     float *dOut = m->buf + size_t(6) * n;
     EdgeBatch b{m->buf, nullptr, nullptr, n, 0, n};
     const int ntiles = (n + kTile - 1) / kTile;
-    const int grid = std::min(ntiles, m->sms * m->fwdBlocksPerSm);
-    forwardKernel<FWD_OUTPUTS><<<grid, 128, kFwdSmem>>>(m->image, b, dOut, nullptr, nullptr, n, m->err);
+    const int grid = std::min((ntiles + kGroups - 1) / kGroups, m->sms * m->fwdBlocksPerSm);
+    forwardKernel<FWD_OUTPUTS><<<grid, 128 * kGroups, kFwdSmem>>>(m->image, b, dOut, nullptr, nullptr, n, m->err);
     MLP_TRY(cudaGetLastError());
     MLP_TRY(cudaMemcpy(out, dOut, size_t(4) * n * sizeof(float), cudaMemcpyDeviceToHost));
     return m->checkErr("forward");
@@ -1123,8 +1228,8 @@ int swe_mlp_solve(swe_mlp *m, int n, const float *edges, float *updates, float *
     uint8_t *dUsed = reinterpret_cast<uint8_t *>(dS + n);
     EdgeBatch b{m->buf, nullptr, nullptr, n, 0, n};
     const int ntiles = (n + kTile - 1) / kTile;
-    const int grid = std::min(ntiles, m->sms * m->fwdBlocksPerSm);
-    forwardKernel<FWD_SOLVE><<<grid, 128, kFwdSmem>>>(m->image, b, dU, dS, dUsed, n, m->err);
+    const int grid = std::min((ntiles + kGroups - 1) / kGroups, m->sms * m->fwdBlocksPerSm);
+    forwardKernel<FWD_SOLVE><<<grid, 128 * kGroups, kFwdSmem>>>(m->image, b, dU, dS, dUsed, n, m->err);
     MLP_TRY(cudaGetLastError());
     MLP_TRY(cudaMemcpy(updates, dU, size_t(4) * n * sizeof(float), cudaMemcpyDeviceToHost));
     MLP_TRY(cudaMemcpy(speed, dS, size_t(n) * sizeof(float), cudaMemcpyDeviceToHost));
@@ -1249,8 +1354,8 @@ cudaError_t launchSurrogateEdges(const DomainDev &d, const swe_mlp *m, const Edg
                                  unsigned long long *used, cudaStream_t s) {
     if (ntiles <= 0) return cudaSuccess;
     if (m) {
-        const int grid = std::min(ntiles, m->sms * m->fwdBlocksPerSm);
-        surrogateEdgeKernel<true><<<grid, 128, kFwdSmem, s>>>(d, m->image, tiles, ntiles, u, used, m->err);
+        const int grid = std::min((ntiles + kGroups - 1) / kGroups, m->sms * m->fwdBlocksPerSm);
+        surrogateEdgeKernel<<<grid, 128 * kGroups, kFwdSmem, s>>>(d, m->image, tiles, ntiles, u, used, m->err);
     } else {
         // the augmented solver alone: as many resident CTAs as registers allow
         // (latency hiding for its long dependency chains), looked up once per device
@@ -1261,11 +1366,11 @@ cudaError_t launchSurrogateEdges(const DomainDev &d, const swe_mlp *m, const Edg
         if (!perSm[dev]) {
             cudaDeviceGetAttribute(&smCount[dev], cudaDevAttrMultiProcessorCount, dev);
             int occ = 0;
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, surrogateEdgeKernel<false>, 128, 0);
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, augEdgeKernel, 128, 0);
             perSm[dev] = std::max(1, occ);
         }
         const int grid = std::min(ntiles, smCount[dev] * perSm[dev]);
-        surrogateEdgeKernel<false><<<grid, 128, 0, s>>>(d, nullptr, tiles, ntiles, u, used, nullptr);
+        augEdgeKernel<<<grid, 128, 0, s>>>(d, tiles, ntiles, u);
     }
     return cudaGetLastError();
 }

@@ -48,7 +48,7 @@ inline std::vector<EdgeTile> buildEdgeTiles(const std::vector<BlockDesc> &blocks
 /// a multiple of 128 its last tile would hold one edge: those blocks' lowest
 /// y-edges (0|1) go to tiles along the row instead (512-row blocks: 8 tiles per
 /// column instead of 9, the edge pass of the augmented solver at 2048^2 144 ->
-/// N us).
+/// 132 us).
 inline std::vector<EdgeTile> buildStepTiles(const std::vector<BlockDesc> &blocks) {
     std::vector<EdgeTile> t;
     for (int k = 0; k < int(blocks.size()); k++) {

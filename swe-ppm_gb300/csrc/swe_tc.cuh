@@ -20,7 +20,7 @@
 // operand of the weight-gradient GEMM (K = edges).
 //
 // Accumulators: M = 128 rows, row r in TMEM lane r, column j in TMEM column
-// base + j (FP32).  Warp w of the CTA reads lanes 32w .. 32w+31.
+// base + j (FP32).  Warp w of the CTA reads lanes 32 (w % 4) .. 32 (w % 4) + 31.
 #pragma once
 
 #include <cstdint>
@@ -105,7 +105,7 @@ __device__ __forceinline__ void fenceSmemForMma() { asm volatile("fence.proxy.as
 
 /// 16 FP32 columns of this thread's TMEM lane, starting at column `col`
 __device__ __forceinline__ void load16(uint32_t tbase, int col, float (&v)[16]) {
-    const uint32_t lane = (threadIdx.x >> 5) * 32u;
+    const uint32_t lane = ((threadIdx.x >> 5) & 3u) * 32u;
     uint32_t r[16];
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
