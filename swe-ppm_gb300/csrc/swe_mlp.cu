@@ -34,6 +34,7 @@
 #include "../../include/swe_gb300.h"
 #include "../../include/swe_gb300_mlp.h"
 #include "swe_device.cuh"
+#include "swe_launch.hpp"
 #include "swe_mlp_launch.hpp"
 #include "swe_sweep.cuh"
 #include "swe_tc.cuh"
@@ -64,15 +65,21 @@ constexpr float kGateTau = 0.25f;     // |strengths - closure| <= tau (|closure|
 constexpr float kMinSpread = 0.5f;    // s2 - s1 >= 0.5 c to use the surrogate
 constexpr float kTrainSpread = 0.1f;  // s2 - s1 < 0.1 c: no gradient
 
-// forward (inference) kernels: kGroups groups of 128 threads, each on a tile of
-// its own, share the CTA's weights.  The features of a group's next tile use
+// forward (inference) kernels: up to kGroups groups of 128 threads, each on a
+// tile of its own, share the CTA's weights.  The features of a group's next tile use
 // its activation buffer (layer 1 has been read before its activations are
 // written), so a group needs 16 KB and 64 TMEM columns: two CTAs of four fill
 // an SM's 512 columns with 32 warps.  CTAs of one group each, with their own
-// 21 KB of weights and a feature buffer, came to 20 warps.
+// 21 KB of weights and a feature buffer, came to 20 warps.  A batch that does
+// not fill the SMs that way takes fewer groups per CTA (fwdGroups).
 constexpr int kGroups = 4;
-constexpr int kFwdAct = kImageSmem, kFwdSmem = kFwdAct + kGroups * kActBytes;
+constexpr int kFwdAct = kImageSmem;
+constexpr int fwdSmem(int groups) { return kFwdAct + groups * kActBytes; }
+constexpr int kFwdSmem = fwdSmem(kGroups);
 constexpr uint32_t kFwdCols = 64;
+/// groups per CTA for a number of tiles: 4 once every SM has work for them, else
+/// 2 or 1, so that tiles spread over the SMs before they share one
+inline int fwdGroups(int ntiles, int sms) { return ntiles > 2 * sms ? kGroups : ntiles > sms ? 2 : 1; }
 // training kernel: shared memory ...
 constexpr int kTrOnes = kImageSmem, kTrX0 = kTrOnes + kOnesBytes, kTrA1 = kTrX0 + kX0Bytes, kTrA2 = kTrA1 + kActBytes,
               kTrA3 = kTrA2 + kActBytes, kTrDZ4 = kTrA3 + kActBytes, kTrDZ = kTrDZ4 + kX0Bytes,
@@ -375,9 +382,10 @@ struct FwdGroup {
 /// a forward CTA's set-up: weights, TMEM columns, a barrier per group
 __device__ __forceinline__ FwdGroup fwdBegin(const uint8_t *image, uint8_t *smem, uint64_t *mbar, uint32_t *tslot, float *sHb) {
     stageImage(image, smem, sHb);
+    const int groups = int(blockDim.x >> 7);
     if (threadIdx.x == 0)
-        for (int g = 0; g < kGroups; g++) tc::mbarInit(mbar + g, 1);
-    if (threadIdx.x < 32) tc::tmemAlloc(tslot, kFwdCols * kGroups);
+        for (int g = 0; g < groups; g++) tc::mbarInit(mbar + g, 1);
+    if (threadIdx.x < 32) tc::tmemAlloc(tslot, kFwdCols * groups);
     tc::fenceSmemForMma();
     tc::fenceBeforeSync();
     __syncthreads();
@@ -405,7 +413,7 @@ __device__ __forceinline__ void fwdEnd(FwdGroup &G, bool ok, uint32_t tslot, int
     }
     tc::fenceBeforeSync();
     __syncthreads();
-    if (threadIdx.x < 32) tc::tmemFree(tslot, kFwdCols * kGroups);
+    if (threadIdx.x < 32) tc::tmemFree(tslot, kFwdCols * (blockDim.x >> 7));
 }
 
 /// edges in structure-of-arrays form: quantity k of edge e at v[k * stride + idx(e)]
@@ -432,7 +440,8 @@ __global__ void __launch_bounds__(128 * kGroups, 2) forwardKernel(const uint8_t 
     FwdGroup G = fwdBegin(image, smem, mbar, &tslot, sHb);
     bool ok = true;
     const int ntiles = (in.count + kTile - 1) / kTile;
-    for (int tile = blockIdx.x * kGroups + G.id; ok && tile < ntiles; tile += gridDim.x * kGroups) {
+    const int groups = int(blockDim.x >> 7);
+    for (int tile = blockIdx.x * groups + G.id; ok && tile < ntiles; tile += gridDim.x * groups) {
         const int i = tile * kTile + G.t;
         const bool valid = i < in.count;
         float q[6] = {1.f, 1.f, 0.f, 0.f, 0.f, 0.f};
@@ -483,11 +492,32 @@ __global__ void __launch_bounds__(128, 1) trainKernel(const uint8_t *image, Edge
     const int t = threadIdx.x;
     uint8_t *sW = smem, *sOnes = smem + kTrOnes, *sX0 = smem + kTrX0, *sDZ4 = smem + kTrDZ4, *sDZ = smem + kTrDZ;
     uint8_t *const act = smem + kTrA1;  // A1, A2, A3
-    stageImage(image, sW, sHb);
+    // what does not depend on the batch before -- the constant operands, the
+    // TMEM columns, the first tile's edges -- comes before the wait for its
+    // Adam step, the weights after it
     for (int i = t; i < kOnesBytes / 4; i += blockDim.x) reinterpret_cast<uint32_t *>(sOnes)[i] = 0x3F803F80u;  // BF16 1.0
     for (int i = t; i < (kTrEnd - kTrDZ4) / 4; i += blockDim.x) reinterpret_cast<uint32_t *>(sDZ4)[i] = 0u;
     if (t == 0) tc::mbarInit(&mbar, 1);
     if (t < 32) tc::tmemAlloc(&tslot, kTrCols);
+    const int ntiles = (in.count + kTile - 1) / kTile;
+    float q[6], T[4];
+    bool valid = false;
+    auto load = [&](int tile) {
+        const int i = tile * kTile + t;
+        valid = i < in.count;
+        q[0] = q[1] = 1.f;
+        q[2] = q[3] = q[4] = q[5] = T[0] = T[1] = T[2] = T[3] = 0.f;
+        if (valid) {
+            const long long e = in.index(i);
+#pragma unroll
+            for (int k = 0; k < 6; k++) q[k] = __ldg(in.v + k * in.stride + e);
+#pragma unroll
+            for (int k = 0; k < 4; k++) T[k] = __ldg(in.targets + k * in.stride + e);
+        }
+    };
+    load(blockIdx.x);
+    pdlWaitAndRelease();
+    stageImage(image, sW, sHb);
     tc::fenceBeforeSync();
     __syncthreads();
     tc::fenceAfterSync();
@@ -496,18 +526,8 @@ __global__ void __launch_bounds__(128, 1) trainKernel(const uint8_t *image, Edge
     uint32_t phase = 0;
     bool ok = true, first = true;
     float lossSum = 0.f;
-    const int ntiles = (in.count + kTile - 1) / kTile;
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const int i = tile * kTile + t;
-        const bool valid = i < in.count;
-        float q[6] = {1.f, 1.f, 0.f, 0.f, 0.f, 0.f}, T[4] = {0.f, 0.f, 0.f, 0.f};
-        if (valid) {
-            const long long e = in.index(i);
-#pragma unroll
-            for (int k = 0; k < 6; k++) q[k] = __ldg(in.v + k * in.stride + e);
-#pragma unroll
-            for (int k = 0; k < 4; k++) T[k] = __ldg(in.targets + k * in.stride + e);
-        }
+        if (!first) load(tile);
         EdgeFeat f;
         edgeFeatures(q[0], q[1], q[2], q[3], q[4], q[5], f);
         storeX0(sX0, t, f.x);
@@ -632,7 +652,7 @@ __global__ void __launch_bounds__(64) reduceAdamKernel(const float *partials, in
                                                        float *m, float *v, float lr, float beta1, float beta2, float eps,
                                                        float bc1, float bc2, uint8_t *image) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i > kNParams) return;
+    // (the training kernel has waited for the step before, which wrote these)
     float mi = 0.f, vi = 0.f, pi = 0.f;
     const bool adam = lr > 0.f && i < kNParams;
     if (adam) {
@@ -640,6 +660,8 @@ __global__ void __launch_bounds__(64) reduceAdamKernel(const float *partials, in
         vi = v[i];
         pi = p[i];
     }
+    pdlWaitAndRelease();
+    if (i > kNParams) return;
     float g = 0.f;
     int c = 0;
     for (; c + 16 <= nparts; c += 16) {
@@ -697,6 +719,56 @@ __global__ void packKernel(const float *p, uint8_t *image) {
     }
 }
 constexpr int kPackThreads = kHid * kInPad + 2 * kHid * kHid + kOutPad * kHid + kBiasFloats;
+
+// ---------------------------------------------------------------------------
+// An epoch's order: the Fisher-Yates shuffle for (i = n-1; i > 0; i--)
+// swap(perm[i], perm[j_i]) with j_i = draw mod (i+1), on the device.
+//
+// Position x holds, just before iteration x, what the last swap into it left
+// there: the value position next(x) held just before iteration next(x), where
+// next(x) is the smallest i > x with j_i = x, or x itself if there is none.  So
+// that value is the end of the chain x, next(x), next(next(x)), ...; and
+// perm[i] is what position j_i held before iteration i: the end of the chain
+// from the smallest i' > i with j_i' = j_i, or j_i itself.  The draws are a
+// counter's hashes, so every position is independent of the others: chains and
+// lists of iterations by target are a dozen links long.  On the host the swaps
+// of 65536 edges took 383 us of an epoch's 675; here about 20 us.
+// ---------------------------------------------------------------------------
+/// the draws of one shuffle: a splitmix64 stream behind state s0
+__device__ __forceinline__ int shuffleTarget(unsigned long long s0, int n, int i) {
+    unsigned long long z = s0 + 0x9E3779B97F4A7C15ull * (unsigned long long)(n - i);
+    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
+    z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
+    return int((z ^ (z >> 31)) % (unsigned long long)(i + 1));
+}
+/// the smallest iteration above i in the list of target x; -1 if there is none
+__device__ __forceinline__ int shuffleAbove(const int *head, const int *link, int x, int i) {
+    int best = -1;
+    for (int k = head[x]; k >= 0; k = link[k])
+        if (k > i && (best < 0 || k < best)) best = k;
+    return best;
+}
+/// lists of iterations by target (head: -1 everywhere)
+__global__ void shuffleListKernel(unsigned long long s0, int n, int *head, int *link) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
+    if (i < n) link[i] = atomicExch(&head[shuffleTarget(s0, n, i)], i);
+}
+__global__ void shuffleNextKernel(int n, const int *head, const int *link, int *next) {
+    const int x = blockIdx.x * blockDim.x + threadIdx.x;
+    if (x < n) next[x] = shuffleAbove(head, link, x, x);
+}
+__global__ void shuffleOrderKernel(unsigned long long s0, int n, const int *head, const int *link, const int *next, int *perm) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int j = i > 0 ? shuffleTarget(s0, n, i) : 0;
+    int x = j == i ? i : shuffleAbove(head, link, j, i);
+    if (x < 0) {
+        x = j;
+    } else {
+        for (int k = next[x]; k >= 0; k = next[k]) x = k;
+    }
+    perm[i] = x;
+}
 
 // ---------------------------------------------------------------------------
 // descriptor self-checks (one CTA): the operand readings the kernels use
@@ -811,7 +883,7 @@ __global__ void __launch_bounds__(128 * kGroups, 2)
     bool ok = true;
     float smax = 0.f;
     unsigned usedLocal = 0;
-    const int worker = blockIdx.x * kGroups + G.id, workers = gridDim.x * kGroups;
+    const int groups = int(blockDim.x >> 7), worker = blockIdx.x * groups + G.id, workers = gridDim.x * groups;
     const int first = int((long long)ntiles * worker / workers);
     const int last = int((long long)ntiles * (worker + 1) / workers);
     int group = -1;
@@ -1062,17 +1134,15 @@ struct swe_mlp {
     int trainBatch(const EdgeBatch &b, float invN, float lr, float *gradDst, float *lossDst) {
         const int ntiles = (b.count + kTile - 1) / kTile;
         const int grid = std::max(1, std::min(ntiles, sms));
-        trainKernel<<<grid, 128, kTrSmem>>>(image, b, invN, partials, err);
-        MLP_TRY(cudaGetLastError());
+        MLP_TRY(launchPdlSmem(trainKernel, dim3(grid), dim3(128), kTrSmem, nullptr, image, b, invN, partials, err));
         float bc1 = 1.f, bc2 = 1.f;
         if (lr > 0.f) {
             adamSteps++;
             bc1 = 1.f - std::pow(0.9f, float(adamSteps));
             bc2 = 1.f - std::pow(0.999f, float(adamSteps));
         }
-        reduceAdamKernel<<<(kNParams + 1 + 63) / 64, 64>>>(partials, grid, gradDst, lossDst, p, m, v, lr, 0.9f, 0.999f, 1e-8f,
-                                                           bc1, bc2, image);
-        MLP_TRY(cudaGetLastError());
+        MLP_TRY(launchPdl(reduceAdamKernel, dim3((kNParams + 1 + 63) / 64), dim3(64), nullptr, partials, grid, gradDst, lossDst,
+                          p, m, v, lr, 0.9f, 0.999f, 1e-8f, bc1, bc2, image));
         return SWE_GPU_OK;
     }
 };
@@ -1210,8 +1280,8 @@ int swe_mlp_forward(swe_mlp *m, int n, const float *edges, float *out) {
     float *dOut = m->buf + size_t(6) * n;
     EdgeBatch b{m->buf, nullptr, nullptr, n, 0, n};
     const int ntiles = (n + kTile - 1) / kTile;
-    const int grid = std::min((ntiles + kGroups - 1) / kGroups, m->sms * m->fwdBlocksPerSm);
-    forwardKernel<FWD_OUTPUTS><<<grid, 128 * kGroups, kFwdSmem>>>(m->image, b, dOut, nullptr, nullptr, n, m->err);
+    const int groups = fwdGroups(ntiles, m->sms), grid = std::min((ntiles + groups - 1) / groups, m->sms * m->fwdBlocksPerSm);
+    forwardKernel<FWD_OUTPUTS><<<grid, 128 * groups, fwdSmem(groups)>>>(m->image, b, dOut, nullptr, nullptr, n, m->err);
     MLP_TRY(cudaGetLastError());
     MLP_TRY(cudaMemcpy(out, dOut, size_t(4) * n * sizeof(float), cudaMemcpyDeviceToHost));
     return m->checkErr("forward");
@@ -1228,8 +1298,8 @@ int swe_mlp_solve(swe_mlp *m, int n, const float *edges, float *updates, float *
     uint8_t *dUsed = reinterpret_cast<uint8_t *>(dS + n);
     EdgeBatch b{m->buf, nullptr, nullptr, n, 0, n};
     const int ntiles = (n + kTile - 1) / kTile;
-    const int grid = std::min((ntiles + kGroups - 1) / kGroups, m->sms * m->fwdBlocksPerSm);
-    forwardKernel<FWD_SOLVE><<<grid, 128 * kGroups, kFwdSmem>>>(m->image, b, dU, dS, dUsed, n, m->err);
+    const int groups = fwdGroups(ntiles, m->sms), grid = std::min((ntiles + groups - 1) / groups, m->sms * m->fwdBlocksPerSm);
+    forwardKernel<FWD_SOLVE><<<grid, 128 * groups, fwdSmem(groups)>>>(m->image, b, dU, dS, dUsed, n, m->err);
     MLP_TRY(cudaGetLastError());
     MLP_TRY(cudaMemcpy(updates, dU, size_t(4) * n * sizeof(float), cudaMemcpyDeviceToHost));
     MLP_TRY(cudaMemcpy(speed, dS, size_t(n) * sizeof(float), cudaMemcpyDeviceToHost));
@@ -1262,13 +1332,14 @@ int swe_mlp_train(swe_mlp *m, int n, const float *edges, const float *targets, i
     if ((rc = m->reserve(size_t(10) * n))) return rc;
     MLP_TRY(cudaMemcpy(m->buf, edges, size_t(6) * n * sizeof(float), cudaMemcpyHostToDevice));
     MLP_TRY(cudaMemcpy(m->buf + size_t(6) * n, targets, size_t(4) * n * sizeof(float), cudaMemcpyHostToDevice));
-    if (size_t(n) > m->permCap) {
+    if (size_t(n) > m->permCap) {  // the order, then the shuffle's lists
         cudaFree(m->perm);
         m->perm = nullptr;
         m->permCap = 0;
-        MLP_TRY(cudaMalloc(&m->perm, size_t(n) * sizeof(int)));
+        MLP_TRY(cudaMalloc(&m->perm, size_t(4) * n * sizeof(int)));
         m->permCap = n;
     }
+    int *head = m->perm + n, *link = head + n, *next = link + n;
     const int nb = (n + batch - 1) / batch;
     if (size_t(nb) * epochs > m->lossCap) {
         cudaFree(m->losses);
@@ -1277,12 +1348,15 @@ int swe_mlp_train(swe_mlp *m, int n, const float *edges, const float *targets, i
         MLP_TRY(cudaMalloc(&m->losses, size_t(nb) * epochs * sizeof(float)));
         m->lossCap = size_t(nb) * epochs;
     }
-    std::vector<int> perm(n);
-    uint64_t s = seed;
+    unsigned long long s = seed;
+    const unsigned tiles = unsigned((n + 255) / 256);
     for (int ep = 0; ep < epochs; ep++) {
-        for (int i = 0; i < n; i++) perm[i] = i;
-        for (int i = n - 1; i > 0; i--) std::swap(perm[i], perm[int(splitmix(s) % uint64_t(i + 1))]);
-        MLP_TRY(cudaMemcpy(m->perm, perm.data(), size_t(n) * sizeof(int), cudaMemcpyHostToDevice));
+        MLP_TRY(cudaMemsetAsync(head, 0xFF, size_t(n) * sizeof(int)));
+        shuffleListKernel<<<tiles, 256>>>(s, n, head, link);
+        shuffleNextKernel<<<tiles, 256>>>(n, head, link, next);
+        shuffleOrderKernel<<<tiles, 256>>>(s, n, head, link, next, m->perm);
+        MLP_TRY(cudaGetLastError());
+        s += 0x9E3779B97F4A7C15ull * (unsigned long long)(n - 1);  // the draws this epoch took
         for (int k = 0; k < nb; k++) {
             const int off = k * batch, cnt = std::min(batch, n - off);
             EdgeBatch b{m->buf, m->buf + size_t(6) * n, m->perm, n, off, cnt};
@@ -1354,8 +1428,8 @@ cudaError_t launchSurrogateEdges(const DomainDev &d, const swe_mlp *m, const Edg
                                  unsigned long long *used, cudaStream_t s) {
     if (ntiles <= 0) return cudaSuccess;
     if (m) {
-        const int grid = std::min((ntiles + kGroups - 1) / kGroups, m->sms * m->fwdBlocksPerSm);
-        surrogateEdgeKernel<<<grid, 128 * kGroups, kFwdSmem, s>>>(d, m->image, tiles, ntiles, u, used, m->err);
+        const int groups = fwdGroups(ntiles, m->sms), grid = std::min((ntiles + groups - 1) / groups, m->sms * m->fwdBlocksPerSm);
+        surrogateEdgeKernel<<<grid, 128 * groups, fwdSmem(groups), s>>>(d, m->image, tiles, ntiles, u, used, m->err);
     } else {
         // the augmented solver alone: as many resident CTAs as registers allow
         // (latency hiding for its long dependency chains), looked up once per device
