@@ -6,14 +6,19 @@
 namespace swegb {
 
 template <int S> static cudaError_t speed(const DomainDev &d, int n, int th, cudaStream_t s, bool pdl) {
-    const auto k = d.semantics == SEM_SPLIT ? speedSplitKernel<S> : sweepKernel<S, SEM_UNSPLIT, false>;
-    if (pdl) return launchPdl(k, dim3(n), dim3(th), s, d);
-    k<<<n, th, 0, s>>>(d);
+    if (d.semantics == SEM_SPLIT) {
+        if (pdl) return launchPdl(speedSplitKernel<S>, dim3(n), dim3(th), s, d);
+        speedSplitKernel<S><<<n, th, 0, s>>>(d);
+        return cudaGetLastError();
+    }
+    if (pdl) return launchPdlSmem(sweepKernel<S, SEM_UNSPLIT, false, false>, dim3(n), dim3(th), sizeof(SweepShared), s, d);
+    sweepKernel<S, SEM_UNSPLIT, false, false><<<n, th, sizeof(SweepShared), s>>>(d);
     return cudaGetLastError();
 }
 template <int S> static cudaError_t update(const DomainDev &d, int n, int th, cudaStream_t s) {
-    return d.semantics == SEM_SPLIT ? launchPdl(sweepKernel<S, SEM_SPLIT, true>, dim3(n), dim3(th), s, d)
-                                    : launchPdl(sweepKernel<S, SEM_UNSPLIT, true>, dim3(n), dim3(th), s, d);
+    return d.semantics == SEM_SPLIT
+               ? launchPdlSmem(sweepKernel<S, SEM_SPLIT, true, false>, dim3(n), dim3(th), sizeof(SweepShared), s, d)
+               : launchPdlSmem(sweepKernel<S, SEM_UNSPLIT, true, false>, dim3(n), dim3(th), sizeof(SweepShared), s, d);
 }
 template <int S> static cudaError_t lastEdge(const DomainDev &d, int ngroups, cudaStream_t s) {
     return launchPdl(lastEdgeKernel<S>, dim3((ngroups + 31) / 32), dim3(32), s, d, ngroups);
@@ -29,17 +34,18 @@ cudaError_t launchUpdateAug(const DomainDev &d, int n, int th, cudaStream_t s) {
     return d.solver == SOLVER_AUGRIE ? update<SOLVER_AUGRIE>(d, n, th, s) : update<SOLVER_HYBRID>(d, n, th, s);
 }
 
-template <class K> static int occ(K kernel, int th) {
+template <class K> static int occ(K kernel, int th, size_t smem = 0) {
     int a = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, kernel, th, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, kernel, th, smem);
     return a;
 }
 
 /// resident CTAs per SM of one pass's kernel
 template <int S> static int occupancy(int sem, bool upd, int th) {
     const bool split = sem == SEM_SPLIT;
-    return upd ? (split ? occ(sweepKernel<S, SEM_SPLIT, true>, th) : occ(sweepKernel<S, SEM_UNSPLIT, true>, th))
-               : (split ? occ(speedSplitKernel<S>, th) : occ(sweepKernel<S, SEM_UNSPLIT, false>, th));
+    return upd ? (split ? occ(sweepKernel<S, SEM_SPLIT, true, false>, th, sizeof(SweepShared))
+                        : occ(sweepKernel<S, SEM_UNSPLIT, true, false>, th, sizeof(SweepShared)))
+               : (split ? occ(speedSplitKernel<S>, th) : occ(sweepKernel<S, SEM_UNSPLIT, false, false>, th, sizeof(SweepShared)));
 }
 
 int occupancyAug(int solver, int sem, bool update, int threads) {

@@ -6,14 +6,26 @@
 namespace swegb {
 
 template <int S> static cudaError_t speed(const DomainDev &d, int n, int th, cudaStream_t s, bool pdl) {
-    const auto k = d.semantics == SEM_SPLIT ? speedSplitKernel<S> : sweepKernel<S, SEM_UNSPLIT, false>;
-    if (pdl) return launchPdl(k, dim3(n), dim3(th), s, d);
-    k<<<n, th, 0, s>>>(d);
+    if (d.semantics == SEM_SPLIT) {
+        if (pdl) return launchPdl(speedSplitKernel<S>, dim3(n), dim3(th), s, d);
+        speedSplitKernel<S><<<n, th, 0, s>>>(d);
+        return cudaGetLastError();
+    }
+    if (pdl) return launchPdlSmem(sweepKernel<S, SEM_UNSPLIT, false, false>, dim3(n), dim3(th), sizeof(SweepShared), s, d);
+    sweepKernel<S, SEM_UNSPLIT, false, false><<<n, th, sizeof(SweepShared), s>>>(d);
     return cudaGetLastError();
 }
-template <int S> static cudaError_t update(const DomainDev &d, int n, int th, cudaStream_t s) {
-    return d.semantics == SEM_SPLIT ? launchPdl(sweepKernel<S, SEM_SPLIT, true>, dim3(n), dim3(th), s, d)
-                                    : launchPdl(sweepKernel<S, SEM_UNSPLIT, true>, dim3(n), dim3(th), s, d);
+template <int S> static cudaError_t update(const DomainDev &d, int n, int th, int groups, cudaStream_t s) {
+    if (groups == kTeamGroups && d.semantics == SEM_UNSPLIT) {
+        const auto k = sweepKernel<S, SEM_UNSPLIT, true, true>;
+        constexpr int smem = kTeamGroups * int(sizeof(SweepShared));
+        const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) return e;
+        return launchPdlSmem(k, dim3(n / kTeamGroups), dim3(th * kTeamGroups), smem, s, d);
+    }
+    return d.semantics == SEM_SPLIT
+               ? launchPdlSmem(sweepKernel<S, SEM_SPLIT, true, false>, dim3(n), dim3(th), sizeof(SweepShared), s, d)
+               : launchPdlSmem(sweepKernel<S, SEM_UNSPLIT, true, false>, dim3(n), dim3(th), sizeof(SweepShared), s, d);
 }
 template <int S> static cudaError_t lastEdge(const DomainDev &d, int ngroups, cudaStream_t s) {
     return launchPdl(lastEdgeKernel<S>, dim3((ngroups + 31) / 32), dim3(32), s, d, ngroups);
@@ -25,8 +37,8 @@ cudaError_t launchSpeedFH(const DomainDev &d, int n, int th, cudaStream_t s, boo
 cudaError_t launchLastEdgeFH(const DomainDev &d, int ngroups, cudaStream_t s) {
     return d.solver == SOLVER_FWAVE ? lastEdge<SOLVER_FWAVE>(d, ngroups, s) : lastEdge<SOLVER_HLLE>(d, ngroups, s);
 }
-cudaError_t launchUpdateFH(const DomainDev &d, int n, int th, cudaStream_t s) {
-    return d.solver == SOLVER_FWAVE ? update<SOLVER_FWAVE>(d, n, th, s) : update<SOLVER_HLLE>(d, n, th, s);
+cudaError_t launchUpdateFH(const DomainDev &d, int n, int th, int groups, cudaStream_t s) {
+    return d.solver == SOLVER_FWAVE ? update<SOLVER_FWAVE>(d, n, th, groups, s) : update<SOLVER_HLLE>(d, n, th, groups, s);
 }
 
 cudaError_t launchSpeedBound(const DomainDev &d, int grid, cudaStream_t s) {
@@ -36,17 +48,18 @@ cudaError_t launchSpeedBound(const DomainDev &d, int grid, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-template <class K> static int occ(K kernel, int th) {
+template <class K> static int occ(K kernel, int th, size_t smem = 0) {
     int a = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, kernel, th, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, kernel, th, smem);
     return a;
 }
 
 /// resident CTAs per SM of one pass's kernel
 template <int S> static int occupancy(int sem, bool upd, int th) {
     const bool split = sem == SEM_SPLIT;
-    return upd ? (split ? occ(sweepKernel<S, SEM_SPLIT, true>, th) : occ(sweepKernel<S, SEM_UNSPLIT, true>, th))
-               : (split ? occ(speedSplitKernel<S>, th) : occ(sweepKernel<S, SEM_UNSPLIT, false>, th));
+    return upd ? (split ? occ(sweepKernel<S, SEM_SPLIT, true, false>, th, sizeof(SweepShared))
+                        : occ(sweepKernel<S, SEM_UNSPLIT, true, false>, th, sizeof(SweepShared)))
+               : (split ? occ(speedSplitKernel<S>, th) : occ(sweepKernel<S, SEM_UNSPLIT, false, false>, th, sizeof(SweepShared)));
 }
 
 int occupancyFH(int solver, int sem, bool update, int threads) {

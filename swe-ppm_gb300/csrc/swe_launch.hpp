@@ -47,7 +47,7 @@ inline cudaError_t launchPdlSmem(void (*k)(P...), dim3 grid, dim3 block, size_t 
 // pdl: the speed pass may be scheduled while the previous kernel finishes; the
 // work list must then be one that no kernel in flight writes
 cudaError_t launchSpeedFH(const DomainDev &d, int nunits, int threads, cudaStream_t s, bool pdl);
-cudaError_t launchUpdateFH(const DomainDev &d, int nunits, int threads, cudaStream_t s);
+cudaError_t launchUpdateFH(const DomainDev &d, int nunits, int threads, int groups, cudaStream_t s);
 // the split step's dt from its last x-edge (SPLIT_DT_LAST_EDGE)
 cudaError_t launchLastEdgeFH(const DomainDev &d, int ngroups, cudaStream_t s);
 // same for the augmented and hybrid solvers
@@ -85,8 +85,10 @@ inline cudaError_t launchLastEdge(const DomainDev &d, int ngroups, cudaStream_t 
     return (d.solver == SOLVER_FWAVE || d.solver == SOLVER_HLLE) ? launchLastEdgeFH(d, ngroups, s)
                                                                  : launchLastEdgeAug(d, ngroups, s);
 }
-inline cudaError_t launchUpdate(const DomainDev &d, int nunits, int threads, cudaStream_t s) {
-    return (d.solver == SOLVER_FWAVE || d.solver == SOLVER_HLLE) ? launchUpdateFH(d, nunits, threads, s)
+/// groups: 1, or kTeamGroups for the f-wave and HLLE unsplit step in CTAs of
+/// that many teams (256 threads each, nunits a multiple of it)
+inline cudaError_t launchUpdate(const DomainDev &d, int nunits, int threads, int groups, cudaStream_t s) {
+    return (d.solver == SOLVER_FWAVE || d.solver == SOLVER_HLLE) ? launchUpdateFH(d, nunits, threads, groups, s)
                                                                  : launchUpdateAug(d, nunits, threads, s);
 }
 

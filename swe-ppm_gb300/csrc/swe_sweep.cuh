@@ -30,6 +30,7 @@
 #pragma once
 
 #include <cstddef>
+#include <type_traits>
 
 #include "swe_device.cuh"
 
@@ -155,38 +156,86 @@ __device__ __forceinline__ bool ltsInSync(const LtsBlock &L) {
            L.received[3] != GL_UNVALID && L.stepSizeCounter <= L.stepSize;
 }
 
+/// The threads that work on one segment: the whole CTA ...
+struct CtaTeam {
+    __device__ __forceinline__ int rank() const { return threadIdx.x; }
+    __device__ __forceinline__ int size() const { return blockDim.x; }
+    __device__ __forceinline__ int worker() const { return blockIdx.x; }
+    __device__ __forceinline__ int workers() const { return gridDim.x; }
+    __device__ __forceinline__ void sync() const { __syncthreads(); }
+    __device__ __forceinline__ bool any(bool v) const { return __syncthreads_or(v); }
+    __device__ __forceinline__ void pace() {}
+};
+
+/// ... or one of four groups of 256 threads of a CTA that fills an SM.  Groups
+/// meet every kPace columns (as long as all of them have columns left): the
+/// warp scheduler favours the warps of some groups, and without it they drift
+/// apart until the last group runs alone on its SM.
+constexpr int kPace = 4, kTeamGroups = 4;
+struct GroupTeam {
+    int left;  // columns up to which meetings are still held
+    /// (broadcast, so that the compiler knows it to be the same in a warp)
+    __device__ __forceinline__ int group() const { return __shfl_sync(0xffffffffu, int(threadIdx.x >> 8), 0); }
+    __device__ __forceinline__ int rank() const { return int(threadIdx.x & 255u); }
+    __device__ __forceinline__ int size() const { return 256; }
+    __device__ __forceinline__ int worker() const { return int(blockIdx.x) * kTeamGroups + id; }
+    __device__ __forceinline__ int workers() const { return int(gridDim.x) * kTeamGroups; }
+    int id;  // group()
+    __device__ __forceinline__ void sync() const { asm volatile("bar.sync %0, 256;" ::"r"(id + 1) : "memory"); }
+    __device__ __forceinline__ bool any(bool v) const {
+        unsigned r;
+        asm volatile("{\n.reg .pred p, q;\nsetp.ne.b32 p, %2, 0;\nbarrier.cta.red.or.pred q, %1, 256, p;\nselp.u32 %0, 1, 0, q;\n}"
+                     : "=r"(r)
+                     : "r"(id + 1), "r"(v ? 1 : 0)
+                     : "memory");
+        return r != 0;
+    }
+    /// the group has `columns` columns to do; sMin: shared, one int per CTA
+    __device__ __forceinline__ void begin(int columns, int *sMin) {
+        if (threadIdx.x == 0) *sMin = 0x7fffffff;
+        __syncthreads();
+        if (rank() == 0) atomicMin(sMin, columns);
+        __syncthreads();
+        left = *sMin / kPace * kPace;
+    }
+    /// one more column is done
+    __device__ __forceinline__ void pace() {
+        if (--left >= 0 && left % kPace == 0) __syncthreads();
+    }
+};
+
 /// Segments of this CTA under local time stepping: the pass's work list
 /// (DomainDev::ltsWork) names the blocks that take part, with the prefix sums
 /// of their (row tile, column) pairs; CTA c takes pairs [total c / grid,
 /// total (c+1) / grid), cut at tile ends and every kMaxTileCols columns.
 /// segment(unit, pairs, block's pairs) runs each piece.  Called by every
 /// thread of the CTA.
-template <bool UPDATE, class Seg>
-__device__ __forceinline__ void ltsSegments(const DomainDev &d, int TY, Seg &&segment) {
+template <bool UPDATE, class Team, class Seg>
+__device__ __forceinline__ void ltsSegments(const DomainDev &d, const Team &team, int *sFound, Seg &&segment) {
+    const int TY = team.size();
     int *W = d.ltsWork;
     const int n = __ldcg(W + (UPDATE ? kLwNUpd : kLwNSpd));
     const long long total = __ldcg(W + (UPDATE ? kLwTotUpd : kLwTotSpd));
     const int *list = lwList(W, d.nblocks, UPDATE);
     const int *pref = lwPrefix(W, d.nblocks, UPDATE);
-    long long pos = total * blockIdx.x / gridDim.x;
-    const long long end = total * (blockIdx.x + 1) / gridDim.x;
+    long long pos = total * team.worker() / team.workers();
+    const long long end = total * (team.worker() + 1) / team.workers();
     if (pos >= end || n <= 0) return;
     // the entry holding pair pos, pref[j] <= pos < pref[j+1], with its block
     // and prefixes: every thread tests its own entries, so the search is one
     // round of loads (a binary search is log2(n) dependent ones)
-    __shared__ int sJ, sK, sP0, sP1;
-    __syncthreads();
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    team.sync();
+    for (int i = team.rank(); i < n; i += TY) {
         const int a = __ldcg(pref + i), b = __ldcg(pref + i + 1), k = __ldcg(list + i);
         if (a <= pos && pos < b) {
-            sJ = i;
-            sK = k;
-            sP0 = a;
-            sP1 = b;
+            sFound[0] = i;
+            sFound[1] = k;
+            sFound[2] = a;
+            sFound[3] = b;
         }
     }
-    __syncthreads();
-    int j = sJ, k = sK, p0 = sP0, p1 = sP1;
+    team.sync();
+    int j = sFound[0], k = sFound[1], p0 = sFound[2], p1 = sFound[3];
     while (pos < end) {
         const BlockDesc &B = d.blocks[k];
         const long long local = pos - p0;
@@ -286,22 +335,22 @@ template <int S> __device__ __forceinline__ float lastEdgeSpeed(const DomainDev 
 ///
 /// A segment adds `count` to the group's arrivals; the pass is complete at
 /// `total` (0: the group's segment count of the static partition).
-template <bool UPDATE>
-__device__ __forceinline__ void segmentDone(const DomainDev &d, GroupState *G, float segMax, float *sRed, int *sLast,
-                                            int cur, unsigned count = 1u, unsigned total = 0u) {
+template <bool UPDATE, class Team>
+__device__ __forceinline__ void segmentDone(const DomainDev &d, const Team &team, GroupState *G, float segMax, float *sRed,
+                                            int *sLast, int cur, unsigned count = 1u, unsigned total = 0u) {
     float m = 0.f;
     if (!UPDATE) m = blockReduceMax(segMax, sRed);
-    __syncthreads();
-    if (threadIdx.x == 0) {
+    team.sync();
+    if (team.rank() == 0) {
         if (!UPDATE) atomicMax(&G->speedBits, __float_as_uint(m));
         const unsigned prev = arriveAcqRel(&G->arrived, count);
         const unsigned need = total ? total : unsigned(UPDATE ? G->unitsUpd : G->units);
         *sLast = (prev + count == need);
     }
-    __syncthreads();
+    team.sync();
     // the group state the last segment writes is read by the next kernel,
     // which starts after this grid completes (or waits for it): no fence
-    if (*sLast && threadIdx.x == 0) {
+    if (*sLast && team.rank() == 0) {
         if (UPDATE) {
             G->arrived = 0u;
             G->time = G->time + G->dt;
@@ -335,8 +384,9 @@ __device__ __forceinline__ void segmentDone(const DomainDev &d, GroupState *G, f
 /// error; non-finite or huge states give +inf (never skipped).
 __device__ __forceinline__ float cellSpeedBound(float h, float hu, float hv) {
     if (h < kDryTol) return 0.f;
-    const float m = fmaxf(fabsf(hu), fabsf(hv));
-    const float w = fmaf(m, __fdividef(1.f, h), kSqrtG * (h * rsqrtf(h)));
+    float r;  // 1 / sqrt(h)
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(h));
+    const float w = fmaf(fmaxf(fabsf(hu), fabsf(hv)), r * r, kSqrtG * (h * r));
     return (w <= FLT_MAX && h < 1e30f) ? w : INFINITY;
 }
 
@@ -414,32 +464,53 @@ static __device__ __noinline__ void pushGhosts(const DomainDev &d, const BlockDe
     }
 }
 
-template <int S, int SEM, bool UPDATE>
-__global__ void __launch_bounds__(kMaxTileRows, 4) sweepKernel(const DomainDev d) {
+/// shared memory of a team of the sweep kernels
+struct SweepShared {
+    float sC[2][5][kMaxTileRows];  // y-direction cell quantities of column x
+    float sR[2][2][kMaxTileRows];  // right-going (h, hv) update into row t
+    float sBot[2][kMaxTileCols];   // right-going update into row y0 (bottom tile edge)
+    float sTop[2][kMaxTileCols];   // left-going update into row yTop (top tile edge)
+    float sRed[kMaxTileRows / 32];
+    int sLast, sFound[4];
+};
+
+template <int S, int SEM, bool UPDATE, bool GROUPED>
+__global__ void __launch_bounds__(GROUPED ? 1024 : kMaxTileRows, GROUPED ? 1 : 4) sweepKernel(const DomainDev d) {
     // the update pass of the f-wave / HLLE unsplit step also records the
     // speed bounds of the bounded speed pass
     constexpr bool BOUNDS = UPDATE && SEM == SEM_UNSPLIT && (S == SOLVER_HLLE || S == SOLVER_FWAVE);
-    __shared__ float sC[2][6][kMaxTileRows];   // y-direction cell quantities of column x
-    __shared__ float sR[2][2][kMaxTileRows];   // right-going (h, hv) update into row t
-    __shared__ float sBot[2][kMaxTileCols];    // right-going update into row y0 (bottom tile edge)
-    __shared__ float sTop[2][kMaxTileCols];    // left-going update into row yTop (top tile edge)
-    __shared__ float sRed[kMaxTileRows / 32];
-    __shared__ int sLast;
+    using Team = typename std::conditional<GROUPED, GroupTeam, CtaTeam>::type;
+    extern __shared__ __align__(16) char sweepSmem[];
+    __shared__ int sMin;
+    Team team;
+    SweepShared *shared = reinterpret_cast<SweepShared *>(sweepSmem);
+    if constexpr (GROUPED) {
+        team.id = team.group();
+        shared += team.id;
+    }
+    auto &sC = shared->sC;
+    auto &sR = shared->sR;
+    auto &sBot = shared->sBot;
+    auto &sTop = shared->sTop;
+    auto &sRed = shared->sRed;
+    int &sLast = shared->sLast;
+    const int t = team.rank(), TY = team.size(), worker = team.worker();
     const bool bounds = BOUNDS && d.tileW != nullptr;
+    const bool lts = SEM == SEM_UNSPLIT && d.lts != nullptr;  // (its work lists come with it)
     // the static partition and the block descriptors are written only when
     // the domain is built (local time stepping's work lists are not: they
     // come from the previous kernel): bring the first segment's into L1 before waiting for the
     // previous kernel.  The update pass also prefetches the segment's first
     // columns into L2 from the buffer the group state names now (a hint only:
     // every value used is loaded after the wait).
-    if (!d.ltsWork) {
-        const int s0 = d.ctaSeg[blockIdx.x];
-        if (s0 < d.ctaSeg[blockIdx.x + 1]) {
+    if (!lts) {
+        const int s0 = d.ctaSeg[worker];
+        if (s0 < d.ctaSeg[worker + 1]) {
             const WorkUnit w0 = d.units[s0];
             const BlockDesc &B0 = d.blocks[w0.block];
-            if (threadIdx.x == 0) prefetchL1(&B0);
+            if (t == 0) prefetchL1(&B0);
             if (UPDATE) {
-                const int y = w0.y0 + int(threadIdx.x);
+                const int y = w0.y0 + t;
                 // through L2 only: no line of the group state may sit in L1
                 // when the reads after the wait come
                 const int c = __ldcg(&d.groups[B0.group].cur);
@@ -453,10 +524,10 @@ __global__ void __launch_bounds__(kMaxTileRows, 4) sweepKernel(const DomainDev d
                 }
                 // the two cells of this thread's boundary y-edge (see below)
                 const int XC0 = w0.x1 - w0.x0;
-                if (int(threadIdx.x) < 2 * XC0) {
-                    const bool top = int(threadIdx.x) >= XC0;
-                    const int k = top ? int(threadIdx.x) - XC0 : int(threadIdx.x);
-                    const int yl = top ? min(w0.y0 + int(blockDim.x) - 1, B0.ny) : w0.y0 - 1;
+                if (t < 2 * XC0) {
+                    const bool top = t >= XC0;
+                    const int k = top ? t - XC0 : t;
+                    const int yl = top ? min(w0.y0 + TY - 1, B0.ny) : w0.y0 - 1;
 #pragma unroll
                     for (int q = 0; q < 4; q++)
                         asm volatile("prefetch.global.L2 [%0];" ::"l"(f[q] + B0.base + size_t(w0.x0 + k) * P + size_t(yl)));
@@ -466,14 +537,16 @@ __global__ void __launch_bounds__(kMaxTileRows, 4) sweepKernel(const DomainDev d
     }
     pdlWaitAndRelease();
 
-    const int t = threadIdx.x, TY = blockDim.x;
     // one segment: rows [wu.y0, wu.y0 + TY) x columns [wu.x0, wu.x1) of a block
     auto segment = [&](const WorkUnit wu, unsigned count, unsigned total) {
         const BlockDesc B = d.blocks[wu.block];
         // local time stepping: block k is dt group k, so the group's loads
         // need not wait for the block descriptor's
-        GroupState *G = d.groups + (d.ltsWork ? wu.block : B.group);
-        if (!groupActive(G)) return;
+        GroupState *G = d.groups + (lts ? wu.block : B.group);
+        if (!groupActive(G)) {
+            for (int x = wu.x0; x < wu.x1; ++x) team.pace();
+            return;
+        }
         const int cur = __ldg(&G->cur);
         const float *__restrict__ H = pick(d.h, cur) + B.base;
         const float *__restrict__ HU = pick(d.hu, cur) + B.base;
@@ -501,7 +574,7 @@ __global__ void __launch_bounds__(kMaxTileRows, 4) sweepKernel(const DomainDev d
         int rimMode = 0;  // 0: pushGhosts, 1: copy, 2: copy with -hv, 3: keep (local time stepping pushes none)
         long long rimGhost = 0;
         int rimPitch = 0;
-        if (UPDATE && rimRow && B.ny > 1 && !d.lts) {
+        if (UPDATE && rimRow && B.ny > 1 && !lts) {
             const int side = (y == 1) ? 2 : 3;
             const int type = B.bnd[side];
             rimGhost = (side == 2) ? 0 : B.ny + 1;
@@ -525,7 +598,7 @@ __global__ void __launch_bounds__(kMaxTileRows, 4) sweepKernel(const DomainDev d
             dtdy = (SEM == SEM_SPLIT) ? dtdx : dt / B.dy;
         }
 
-        __syncthreads();  // shared buffers of the previous segment are free
+        team.sync();  // shared buffers of the previous segment are free
         // the tile's bottom (y0-1|y0) and top (yTop|yTop+1) y-edges of every column
         for (int i = t; i < 2 * XC; i += TY) {
             const bool top = i >= XC;
@@ -587,11 +660,9 @@ __global__ void __launch_bounds__(kMaxTileRows, 4) sweepKernel(const DomainDev d
                             hn = oldH - (dtdx * sxH + dtdy * syH);
                             hun = oldHU - dtdx * sxHU;
                             hvn = oldHV - dtdy * syHV;
-                            if (hn < 0.f) {
-                                hn = 0.f; hun = 0.f; hvn = 0.f;
-                            } else if (hn < 0.1f) {
-                                hun = 0.f; hvn = 0.f;
-                            }
+                            hun = hn < 0.1f ? 0.f : hun;
+                            hvn = hn < 0.1f ? 0.f : hvn;
+                            hn = hn < 0.f ? 0.f : hn;
                         } else {
                             const float sxH = aL + pendH, sxHU = auL + pendHU;
                             const float hStar = oldH - dtdx * sxH;
@@ -615,7 +686,7 @@ __global__ void __launch_bounds__(kMaxTileRows, 4) sweepKernel(const DomainDev d
                             HVO[o] = hvn;
                             // no ghost pushes under local time stepping: the
                             // next check carries the ring over and rebuilds it
-                            if (!d.lts && (x - 1 == 1 || x - 1 == B.nx || rimRow)) {
+                            if (!lts && (x - 1 == 1 || x - 1 == B.nx || rimRow)) {
                                 if (rimMode != 0 && x - 1 != 1 && x - 1 != B.nx) {
                                     const long long g = rimGhost + (long long)(x - 1) * rimPitch;
                                     if (rimMode == 3) {
@@ -648,12 +719,13 @@ __global__ void __launch_bounds__(kMaxTileRows, 4) sweepKernel(const DomainDev d
             if (x >= x0 && x < x1) {
                 const int buf = x & 1;
                 sC[buf][0][t] = cy.h; sC[buf][1][t] = cy.hn; sC[buf][2][t] = cy.b;
-                sC[buf][3][t] = cy.u; sC[buf][4][t] = cy.sq; sC[buf][5][t] = cy.c;
-                __syncthreads();
+                sC[buf][3][t] = cy.u; sC[buf][4][t] = cy.sq;
+                team.sync();
                 float bLh = 0.f, bLhv = 0.f;
                 if (active && y < yTop) {
+                    const float upSq = sC[buf][4][t + 1];
                     const Cell up = makeCell(sC[buf][0][t + 1], sC[buf][1][t + 1], sC[buf][2][t + 1],
-                                             sC[buf][3][t + 1], sC[buf][4][t + 1], sC[buf][5][t + 1]);
+                                             sC[buf][3][t + 1], upSq, kSqrtG * upSq);
                     if (UPDATE) {
                         float bR, bRhv, s;
                         edgeSolve<S, true>(cy, up, bLh, bR, bLhv, bRhv, s);
@@ -664,7 +736,7 @@ __global__ void __launch_bounds__(kMaxTileRows, 4) sweepKernel(const DomainDev d
                     }
                 }
                 if (UPDATE) {
-                    __syncthreads();
+                    team.sync();
                     if (active) {
                         if (y == yTop) {
                             bLh = sTop[0][x - x0];
@@ -682,27 +754,37 @@ __global__ void __launch_bounds__(kMaxTileRows, 4) sweepKernel(const DomainDev d
                         oldH = ch; oldHU = chu; oldHV = chv;
                     }
                 }
+                team.pace();
             }
         }
-        if (UPDATE && __syncthreads_or(bad) && t == 0) atomicOr(&G->status, 2);
-        segmentDone<UPDATE>(d, G, smax, sRed, &sLast, cur, count, total);
+        if (UPDATE && team.any(bad) && t == 0) atomicOr(&G->status, 2);
+        segmentDone<UPDATE>(d, team, G, smax, sRed, &sLast, cur, count, total);
     };
-    if (d.ltsWork) {
-        ltsSegments<UPDATE>(d, TY, segment);
+    if (lts) {
+        if constexpr (GROUPED) {
+            const long long all = __ldcg(d.ltsWork + (UPDATE ? kLwTotUpd : kLwTotSpd));
+            team.begin(int(all * (worker + 1) / team.workers() - all * worker / team.workers()), &sMin);
+        }
+        ltsSegments<UPDATE>(d, team, shared->sFound, segment);
         if (UPDATE) {
             // the update pass's last CTA ends the iteration
             __syncthreads();
-            if (t == 0)
-                sLast = arriveAcqRel(reinterpret_cast<unsigned *>(d.ltsWork + kLwArrUpd), 1u) + 1u == gridDim.x;
+            if (threadIdx.x == 0)
+                sMin = arriveAcqRel(reinterpret_cast<unsigned *>(d.ltsWork + kLwArrUpd), 1u) + 1u == gridDim.x;
             __syncthreads();
-            if (sLast) {
-                if (t == 0) d.ltsWork[kLwArrUpd] = 0;
+            if (sMin) {
+                if (threadIdx.x == 0) d.ltsWork[kLwArrUpd] = 0;
                 ltsEndIteration(d);
             }
         }
     } else {
-        const int segEnd = d.ctaSeg[blockIdx.x + 1];
-        for (int seg = d.ctaSeg[blockIdx.x]; seg < segEnd; ++seg) segment(d.units[seg], 1u, 0u);
+        const int segBegin = d.ctaSeg[worker], segEnd = d.ctaSeg[worker + 1];
+        if constexpr (GROUPED) {
+            int columns = 0;
+            for (int seg = segBegin; seg < segEnd; ++seg) columns += d.units[seg].x1 - d.units[seg].x0;
+            team.begin(columns, &sMin);
+        }
+        for (int seg = segBegin; seg < segEnd; ++seg) segment(d.units[seg], 1u, 0u);
     }
 }
 
@@ -742,7 +824,7 @@ template <int S> __global__ void __launch_bounds__(kMaxTileRows) speedSplitKerne
                 prev = c;
             }
         }
-        segmentDone<false>(d, G, smax, sRed, &sLast, cur);
+        segmentDone<false>(d, CtaTeam{}, G, smax, sRed, &sLast, cur);
     }
 }
 
