@@ -16,9 +16,14 @@
 //  - Each thread owns two consecutive rows of a tile, computed as packed
 //    pairs (f32x2 add / mul / fma), and marches along x.  The x-edge (x-1|x)
 //    uses the previous column kept in registers, the y-edges the thread's
-//    own rows and the staged row above them.  The right-going part of a
-//    thread's top y-edge reaches the thread above by a shuffle; lane 0
-//    solves the warp's bottom y-edge itself.
+//    own rows and the staged rows above and below them.  Every lane solves
+//    its bottom y-edge itself, although the lane below has solved it as its
+//    top one: the warp issues it for lane 0 anyway, and without the branch
+//    around lane 0 and the shuffle after it the edge runs between the others
+//    (2048^2, back to back: 37.4 -> 34.8 us a step, with the masks of partial
+//    tiles as selects, not branches; warps in flight and latency bound the kernel).
+//    Where a warp solves its edges again (dry cells, supercritical edges),
+//    only lane 0 does the bottom one and the shuffle gives the others theirs.
 //  - The next step's maximum wave speed (computeNumericalFluxes :391-456 on
 //    Q^{n+1}) is evaluated while Q^{n+1} is produced: edges between two cells
 //    of the segment as soon as both exist, edges to a ghost from the boundary
@@ -113,19 +118,21 @@ __device__ __forceinline__ FQ makeFQ(float h, float hn, float eta, float ih, flo
     q.h = h;
     q.hn = hn;
     q.eta = eta;
-    q.u = hn * ih;
+    q.u = __fmul_rn(hn, ih);
     q.sq = sq;
-    q.m = hn * q.u;
-    q.lo = q.u - c;
-    q.hi = q.u + c;
+    q.m = __fmul_rn(hn, q.u);
+    q.lo = __fsub_rn(q.u, c);
+    q.hi = __fadd_rn(q.u, c);
     return q;
 }
 
-/// the same from raw values (one reciprocal square root)
+/// the same from raw values (one reciprocal square root).  Every operation of
+/// the single-edge forms is rounded by itself, as the packed ones are: an edge
+/// that two lanes solve, one in each form, gives both the same bits.
 __device__ __forceinline__ FQ rawFQ(float h, float hn, float b) {
     const float r = aRsqrt(h);
-    const float sq = h * r;
-    return makeFQ(h, hn, h + b, r * r, sq, kSqrtG * sq);
+    const float sq = __fmul_rn(h, r);
+    return makeFQ(h, hn, __fadd_rn(h, b), __fmul_rn(r, r), sq, __fmul_rn(kSqrtG, sq));
 }
 
 __device__ __forceinline__ void routeFast(float s, float zh, float zhu, float &hL, float &hR, float &huL, float &huR) {
@@ -153,32 +160,32 @@ __device__ __forceinline__ void routeFast(float s, float zh, float zhu, float &h
 template <int S, bool GENERAL>
 __device__ __forceinline__ void waves(const FQ &L, const FQ &R, float &aL, float &aR, float &auL, float &auR,
                                       float &sub) {
-    const float rs = aRcp(L.sq + R.sq);
-    const float uRoe = fmaf(L.u, L.sq, R.u * R.sq) * rs;
-    const float ghs = kHalfG * (L.h + R.h);
+    const float rs = aRcp(__fadd_rn(L.sq, R.sq));
+    const float uRoe = __fmul_rn(fmaf(L.u, L.sq, __fmul_rn(R.u, R.sq)), rs);
+    const float ghs = __fmul_rn(kHalfG, __fadd_rn(L.h, R.h));
     const float cRoe = aSqrt(ghs);
-    float s1 = uRoe - cRoe, s2 = uRoe + cRoe;
+    float s1 = __fsub_rn(uRoe, cRoe), s2 = __fadd_rn(uRoe, cRoe);
     if (S == SOLVER_HLLE) {
         s1 = fminf(L.lo, s1);
         s2 = fmaxf(R.hi, s2);
     }
-    const float df1 = R.hn - L.hn;
-    const float df2 = fmaf(ghs, R.eta - L.eta, R.m - L.m);
-    const float rd = aRcp(s2 - s1);
-    const float b1 = fmaf(s2, df1, -df2) * rd;
-    const float b2 = fmaf(-s1, df1, df2) * rd;
+    const float df1 = __fsub_rn(R.hn, L.hn);
+    const float df2 = fmaf(ghs, __fsub_rn(R.eta, L.eta), __fsub_rn(R.m, L.m));
+    const float rd = aRcp(__fsub_rn(s2, s1));
+    const float b1 = __fmul_rn(fmaf(s2, df1, -df2), rd);
+    const float b2 = __fmul_rn(fmaf(-s1, df1, df2), rd);
     if (GENERAL) {
         aL = 0.f;
         aR = 0.f;
         auL = 0.f;
         auR = 0.f;
-        routeFast(s1, b1, b1 * s1, aL, aR, auL, auR);
-        routeFast(s2, b2, b2 * s2, aL, aR, auL, auR);
+        routeFast(s1, b1, __fmul_rn(b1, s1), aL, aR, auL, auR);
+        routeFast(s2, b2, __fmul_rn(b2, s2), aL, aR, auL, auR);
     } else {
         aL = b1;
-        auL = b1 * s1;
+        auL = __fmul_rn(b1, s1);
         aR = b2;
-        auR = b2 * s2;
+        auR = __fmul_rn(b2, s2);
         sub = fminf(sub, fminf(-s1, s2));
     }
 }
@@ -642,14 +649,12 @@ __global__ void __launch_bounds__(kMaxTileRows / (2 * NP), MINB) fastStepKernel(
                 uh = sl[i0 + R];
                 uhv = sl[2 * kSlice + i0 + R];
                 ub = sl[3 * kSlice + i0 + R];
-                if (lane == 0) {  // the cell below the warp's first row
-                    lh = sl[i0 - 1];
-                    lhv = sl[2 * kSlice + i0 - 1];
-                    lb = sl[3 * kSlice + i0 - 1];
-                }
+                // the cell below this lane's first row
+                lh = sl[i0 - 1];
+                lhv = sl[2 * kSlice + i0 - 1];
+                lb = sl[3 * kSlice + i0 - 1];
             }
-            // A. this thread's cells of column x, the cell above its rows and
-            // (lane 0) the one below
+            // A. this thread's cells of column x, the cells above and below its rows
             FQ2 cx[NP], cy[NP];
 #pragma unroll
             for (int q = 0; q < NP; q++) {
@@ -662,7 +667,7 @@ __global__ void __launch_bounds__(kMaxTileRows / (2 * NP), MINB) fastStepKernel(
             FQ up{}, low{};
             if (YCOL) {
                 up = rawFQ(uh, uhv, ub);
-                if (lane == 0) low = rawFQ(lh, lhv, lb);
+                low = rawFQ(lh, lhv, lb);
             }
             // the strip's values are in use, so its reads are complete:
             // release it.  The slot's last releaser refills it; lane 0 reads
@@ -688,8 +693,8 @@ __global__ void __launch_bounds__(kMaxTileRows / (2 * NP), MINB) fastStepKernel(
                 ++rnd;
             }
             // B. x-edges (x-1 | x) and the y-edges between this thread's rows
-            // and from its last row to the staged row above (lane 0: also the
-            // one below its first row), all taken as wet and subsonic first
+            // and to the staged rows above and below, all taken as wet and
+            // subsonic first
             float2 aLx[NP], aRx[NP], auLx[NP], auRx[NP], aLy[NP], aRy[NP], auLy[NP], auRy[NP];
             float sub = 3.0e38f, minh = 3.0e38f;
 #pragma unroll
@@ -701,23 +706,21 @@ __global__ void __launch_bounds__(kMaxTileRows / (2 * NP), MINB) fastStepKernel(
                     minh = fminf(minh, fminf(px[q].h.x, px[q].h.y));
                 }
             }
-            float lowRh = 0.f, lowRhv = 0.f;
+            float lowRh = 0.f, lowRhv = 0.f, subLow = 3.0e38f;
             if (YCOL) {
 #pragma unroll
                 for (int q = 0; q < NP; q++)
                     waves2<S>(cy[q], pairFQ(laneY(cy[q]), q + 1 < NP ? laneX(cy[(q + 1) % NP]) : up), aLy[q], aRy[q],
                               auLy[q], auRy[q], sub);
                 minh = fminf(minh, up.h);
-                if (lane == 0) {
-                    float dl, dlv;
-                    waves<S, false>(low, laneX(cy[0]), dl, lowRh, dlv, lowRhv, sub);
-                    minh = fminf(minh, low.h);
-                }
+                float dl, dlv;
+                waves<S, false>(low, laneX(cy[0]), dl, lowRh, dlv, lowRhv, subLow);
             }
             // C. a lane with a dry cell or an edge that is not subsonic solves
             // its edges again in full (rare: shorelines, fronts)
             if (XCOL || YCOL) {
-                const bool redo = minh < kDryTol || !(sub > kZeroTol);
+                bool redo = minh < kDryTol || !(sub > kZeroTol);
+                if (YCOL) redo = redo || (lane == 0 && (low.h < kDryTol || !(subLow > kZeroTol)));
                 if (__any_sync(FULL, redo)) {
                     if (redo) {
                         if (XCOL) {
@@ -749,6 +752,14 @@ __global__ void __launch_bounds__(kMaxTileRows / (2 * NP), MINB) fastStepKernel(
                             }
                         }
                     }
+                    if (YCOL) {  // the lane below has solved the other lanes' bottom edges
+                        const float pH = __shfl_up_sync(FULL, aRy[NP - 1].y, 1);
+                        const float pHV = __shfl_up_sync(FULL, auRy[NP - 1].y, 1);
+                        if (lane != 0) {
+                            lowRh = pH;
+                            lowRhv = pHV;
+                        }
+                    }
                 }
             }
             // D. cells (x-1, y): Q^{n+1} with the dry clamp, and their part
@@ -761,12 +772,7 @@ __global__ void __launch_bounds__(kMaxTileRows / (2 * NP), MINB) fastStepKernel(
                     hn[q] = sub2(px[q].h, fma2(dtdx, add2(pendH[q], aLx[q]), mul2(dtdy, syH[q])));
                     hun[q] = sub2(px[q].hn, mul2(dtdx, add2(pendHU[q], auLx[q])));
                     hvn[q] = sub2(oldHV[q], mul2(dtdy, syHV[q]));
-                    if (fullTile) {
-                        hsum = add2(hsum, hn[q]);
-                    } else {
-                        hsum.x += 2 * q < nAct ? hn[q].x : 0.f;
-                        hsum.y += 2 * q + 1 < nAct ? hn[q].y : 0.f;
-                    }
+                    hsum = add2(hsum, make_float2(2 * q < nAct ? hn[q].x : 0.f, 2 * q + 1 < nAct ? hn[q].y : 0.f));
                     hun[q].x = (hn[q].x < 0.1f) ? 0.f : hun[q].x;
                     hvn[q].x = (hn[q].x < 0.1f) ? 0.f : hvn[q].x;
                     hun[q].y = (hn[q].y < 0.1f) ? 0.f : hun[q].y;
@@ -799,13 +805,8 @@ __global__ void __launch_bounds__(kMaxTileRows / (2 * NP), MINB) fastStepKernel(
                         const float2 vmax = make_float2(fmaxf(fabsf(hun[q].x), fabsf(hvn[q].x)),
                                                         fmaxf(fabsf(hun[q].y), fabsf(hvn[q].y)));
                         const float2 w = fma2(vmax, mul2(rn[q], rn[q]), mul2(pk(kSqrtG), mul2(hn[q], rn[q])));
-                        if (fullTile) {
-                            wmax = fmaxf(wmax, fmaxf(w.x, w.y));
-                            hmax = fmaxf(hmax, fmaxf(hn[q].x, hn[q].y));
-                        } else {
-                            wmax = fmaxf(wmax, fmaxf(2 * q < nAct ? w.x : 0.f, 2 * q + 1 < nAct ? w.y : 0.f));
-                            hmax = fmaxf(hmax, fmaxf(2 * q < nAct ? hn[q].x : 0.f, 2 * q + 1 < nAct ? hn[q].y : 0.f));
-                        }
+                        wmax = fmaxf(wmax, fmaxf(2 * q < nAct ? w.x : 0.f, 2 * q + 1 < nAct ? w.y : 0.f));
+                        hmax = fmaxf(hmax, fmaxf(2 * q < nAct ? hn[q].x : 0.f, 2 * q + 1 < nAct ? hn[q].y : 0.f));
                     }
                 } else {
                     // f-wave: x-edges (x-2 | x-1), the y-edges between this
@@ -880,13 +881,11 @@ __global__ void __launch_bounds__(kMaxTileRows / (2 * NP), MINB) fastStepKernel(
                 }
             }
             if (YCOL) {
-                // y-sums of column x: the first row's bottom edge from the
-                // lane below (lane 0: its own), the rest from this lane's edges
-                const float pH = __shfl_up_sync(FULL, aRy[NP - 1].y, 1), pHV = __shfl_up_sync(FULL, auRy[NP - 1].y, 1);
+                // y-sums of column x
 #pragma unroll
                 for (int q = 0; q < NP; q++) {
-                    const float bH = q == 0 ? (lane == 0 ? lowRh : pH) : aRy[(q + NP - 1) % NP].y;
-                    const float bHV = q == 0 ? (lane == 0 ? lowRhv : pHV) : auRy[(q + NP - 1) % NP].y;
+                    const float bH = q == 0 ? lowRh : aRy[(q + NP - 1) % NP].y;
+                    const float bHV = q == 0 ? lowRhv : auRy[(q + NP - 1) % NP].y;
                     syH[q] = add2(make_float2(bH, aRy[q].x), aLy[q]);
                     syHV[q] = add2(make_float2(bHV, auRy[q].x), auLy[q]);
                     oldHV[q] = chv[q];
