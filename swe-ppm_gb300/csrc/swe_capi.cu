@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -2286,6 +2287,7 @@ constexpr int kNoAllocMaxDevices = 64;
 struct NoAllocScratch {
     GroupState group;
     BlockDesc block;
+    small::Sync sync;
     WorkUnit units[kNoAllocMaxUnits];
     int ctaSeg[kNoAllocMaxUnits + 1];
 };
@@ -2320,6 +2322,20 @@ int noallocScratch(int device, NoAllocScratch **out) {
     return SWE_GPU_OK;
 }
 
+/// columns per CTA with which all CTAs of a block's step are resident at once;
+/// 0 where they never are.  The capacities are the device's, looked up once.
+int noallocSmallCols(int device, int solver, int tileRows, long long rowTiles, int nx) {
+    static std::atomic<int> known[kNoAllocMaxDevices][5][3][kMaxTileRows / 32];  // capacity + 1
+    if (device < 0 || device >= kNoAllocMaxDevices) return 0;
+    for (int i = 0, cols = 1; cols <= (solver == SWE_SOLVER_AUGRIE ? 1 : small::kMaxCols); i++, cols *= 2) {
+        std::atomic<int> &k = known[device][solver][i][tileRows / 32 - 1];
+        int cap = k.load(std::memory_order_relaxed) - 1;
+        if (cap < 0) k.store((cap = small::capacity(solver, cols, tileRows)) + 1, std::memory_order_relaxed);
+        if (rowTiles * ((nx + cols - 1) / cols) <= cap) return cols;
+    }
+    return 0;
+}
+
 /// writes the block descriptor and work list, clears the control block and
 /// sets the input's ghost ring (setGhostLayer); the ring needs nothing of the
 /// scratch, so one launch does both
@@ -2333,6 +2349,7 @@ __global__ void noallocSetupKernel(NoAllocScratch *s, DomainDev d, BlockDesc b, 
         g.target = INFINITY;
         s->group = g;
         s->block = b;
+        s->sync = small::Sync{0u, 0u, 0ull, nunits, 0};
     }
     const int xChunks = (b.nx + tileCols - 1) / tileCols;
     for (int u = i; u < nunits; u += gridDim.x * blockDim.x) {
@@ -2378,7 +2395,14 @@ extern "C" int swe_gpu_step_block_noalloc(int solver, int semantics, int nx, int
     // the call included).  Where the GPU is full, segments stay at 32 columns:
     // shorter ones solve more edges twice.
     const int tileCols = int(std::max(1LL, std::min(32LL, (rowTiles * nx + 4LL * sms - 1) / (4LL * sms))));
-    const long long nunits = rowTiles * ((nx + tileCols - 1) / tileCols);
+    // A block whose unsplit step fits one cooperative launch (as a small
+    // domain's, swe_small.cu) takes that in the place of the two passes, a
+    // launch less and every edge solved once: 128^2 HLLE 20.6 -> 15.5 us, 424 x
+    // 26 augmented 34.9 -> 22.5, 1200 x 256 f-wave 29.7 -> 23.7 (a call each).
+    // It gains up to its limit, the CTAs that are resident at once.
+    const int smallCols = semantics == SWE_SEMANTICS_UNSPLIT ? noallocSmallCols(device, solver, tileRows, rowTiles, nx) : 0;
+    const int cols = smallCols ? smallCols : tileCols;
+    const long long nunits = rowTiles * ((nx + cols - 1) / cols);
     NoAllocScratch *scr = nullptr;
     int rc = noallocScratch(device, &scr);
     if (rc) return rc;
@@ -2422,11 +2446,16 @@ extern "C" int swe_gpu_step_block_noalloc(int solver, int semantics, int nx, int
     };
     const int threads = 128;
     const long long setupItems = std::max<long long>(2LL * nx + 2LL * ny + 4, nunits);
-    noallocSetupKernel<<<unsigned((setupItems + threads - 1) / threads), threads, 0, s>>>(scr, d, B, tileRows, tileCols,
+    noallocSetupKernel<<<unsigned((setupItems + threads - 1) / threads), threads, 0, s>>>(scr, d, B, tileRows, cols,
                                                                                        int(nunits));
     if ((rc = check(cudaGetLastError(), "set-up kernel"))) return rc;
-    if ((rc = check(launchSpeed(d, int(nunits), tileRows, s, false), "speed pass"))) return rc;
-    if ((rc = check(launchUpdate(d, int(nunits), tileRows, 1, s), "update pass"))) return rc;
+    if (smallCols) {
+        rc = check(small::launch(d, scr->units, int(nunits), &scr->sync, 1, smallCols, tileRows, s), "step");
+        if (rc) return rc;
+    } else {
+        if ((rc = check(launchSpeed(d, int(nunits), tileRows, s, false), "speed pass"))) return rc;
+        if ((rc = check(launchUpdate(d, int(nunits), tileRows, 1, s), "update pass"))) return rc;
+    }
     if (dt_out) {
         if ((rc = check(cudaMemcpyAsync(dt_out, &scr->group.dt, sizeof(float), cudaMemcpyDeviceToHost, s), "dt copy")))
             return rc;
