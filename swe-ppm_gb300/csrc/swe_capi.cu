@@ -271,6 +271,8 @@ struct swe_gpu_domain {
     int maxCols = 0;              // max nx+2 over blocks
     cudaGraphExec_t graph = nullptr;
     int graphSteps = 0;
+    // small domains, in the place of the graph: decided by the first swe_gpu_advance
+    bool smallPrimed = false, smallRing = false, smallStale = false;
     // swe_gpu_advance: the groups' states at its start and after each batch of
     // steps in flight (pinned), the events that mark their copies, and the
     // clock and dt it saw last
@@ -500,7 +502,18 @@ int enqueueStep(swe_gpu_domain *D) {
     return enqueueUpdate(D);
 }
 
-/// `n` steps; the steps of a small domain in launches of at most 256
+/// `n` steps of a small domain, in launches of at most kSmallSteps
+int enqueueSmall(swe_gpu_domain *D, int n) {
+    for (int done = 0; done < n; done += kSmallSteps) {
+        CUDA_TRY(small::launch(D->dev, D->dUnitsS, int(D->unitsS.size()), D->dSync, std::min(n - done, kSmallSteps),
+                               D->smallCols, D->tileRows, D->stream));
+        D->launches++;
+        D->ghostsValid = true;
+    }
+    return SWE_GPU_OK;
+}
+
+/// `n` steps
 int enqueueSteps(swe_gpu_domain *D, int n) {
     if (!D->smallCols) {
         for (int i = 0; i < n; i++) {
@@ -513,13 +526,7 @@ int enqueueSteps(swe_gpu_domain *D, int n) {
         int rc = enqueueGhost(D, 0);
         if (rc) return rc;
     }
-    for (int done = 0; done < n; done += kSmallSteps) {
-        CUDA_TRY(small::launch(D->dev, D->dUnitsS, int(D->unitsS.size()), D->dSync, std::min(n - done, kSmallSteps),
-                               D->smallCols, D->tileRows, D->stream));
-        D->launches++;
-        D->ghostsValid = true;
-    }
-    return SWE_GPU_OK;
+    return enqueueSmall(D, n);
 }
 
 /// one inner iteration of local time stepping (see swe_lts.cu): check
@@ -1627,7 +1634,16 @@ int swe_gpu_advance(swe_gpu_domain *dom, float t_end, int max_steps, int *steps_
         int rc0 = enqueueFastPrologue(dom);
         if (rc0) return rc0;
     }
-    if (!dom->graph) {  // capture `batch` steps once; replays are identical
+    // A small domain's steps need no graph, many go out in one launch (256^2,
+    // 17 steps: 158 -> 152 us a call, 128 steps 1056 -> 963).  Whether batches of 16 and more set a stale ghost ring
+    // first is decided at the first call, as the capture below does it.
+    const bool direct = dom->smallCols > 0;
+    if (direct && !dom->smallPrimed) {
+        dom->smallPrimed = true;
+        dom->smallRing = dom->smallStale = !dom->ghostsValid;
+        dom->ghostsValid = true;
+    }
+    if (!direct && !dom->graph) {  // capture `batch` steps once; replays are identical
         cudaGraph_t g;
         CUDA_TRY(cudaStreamBeginCapture(dom->stream, cudaStreamCaptureModeThreadLocal));
         int rc = SWE_GPU_OK;
@@ -1677,8 +1693,16 @@ int swe_gpu_advance(swe_gpu_domain *dom, float t_end, int max_steps, int *steps_
         while (queued < max_steps && ahead < kAdvanceAhead &&
                (ahead == 0 || double(seenTime) + double(seenDt) * (queued - seenQueued) < double(t_end))) {
             if (ahead > 0 && !(seenDt > 0.f)) break;
-            const int n = std::min(max_steps - queued, dom->graphSteps);
-            if (n == dom->graphSteps) {
+            const int n = std::min(max_steps - queued, direct ? kSmallSteps : dom->graphSteps);
+            if (direct && n >= batch) {
+                if (dom->smallRing && (dom->smallStale || !dom->ghostsValid)) {
+                    rc = enqueueGhost(dom, 0);
+                    if (rc) return rc;
+                    dom->smallStale = false;
+                }
+                rc = enqueueSmall(dom, n);
+                if (rc) return rc;
+            } else if (!direct && n == dom->graphSteps) {
                 CUDA_TRY(cudaGraphLaunch(dom->graph, dom->stream));
                 dom->launches += dom->graphKernels;
             } else {
@@ -1911,6 +1935,7 @@ int swe_gpu_retile(swe_gpu_domain *dom, int tile_rows, int tile_cols) {
     if (dom->graph) cudaGraphExecDestroy(dom->graph);
     if (dom->ltsGraph) cudaGraphExecDestroy(dom->ltsGraph);
     dom->graph = nullptr;
+    dom->smallPrimed = false;
     dom->ltsGraph = nullptr;
     return SWE_GPU_OK;
 }
