@@ -2356,7 +2356,7 @@ int noallocSmallCols(int device, int solver, int tileRows, long long rowTiles, i
         std::atomic<int> &k = known[device][solver][i][tileRows / 32 - 1];
         int cap = k.load(std::memory_order_relaxed) - 1;
         if (cap < 0) k.store((cap = small::capacity(solver, cols, tileRows)) + 1, std::memory_order_relaxed);
-        if (rowTiles * ((nx + cols - 1) / cols) <= cap) return cols;
+        if (rowTiles * ((nx + cols - 1) / cols) <= std::min(cap, kNoAllocMaxUnits)) return cols;
     }
     return 0;
 }

@@ -1,6 +1,7 @@
 """The allocation-free block step in one cooperative launch (blocks whose CTAs
 are all resident at once) against a domain's two-pass step, bit for bit: one,
-two and four columns per CTA, blocks just within and just beyond the limit,
+two and four columns per CTA, blocks just within and just beyond the limit
+(of resident CTAs, and of the unit table),
 one-cell blocks, and a captured call replayed on a second state."""
 import numpy as np
 import pytest
@@ -37,7 +38,7 @@ def two_pass(swe, solver, nx, ny, st):
 
 @pytest.mark.parametrize("solver,nx,ny", [
     (4, 1, 1), (4, 33, 31), (1, 608, 256), (1, 609, 256), (4, 1217, 255), (3, 300, 300), (2, 424, 26),
-    (4, 1824, 250), (4, 1900, 256), (1, 2500, 100),
+    (4, 1824, 250), (4, 1900, 256), (1, 2500, 100), (4, 4096, 20), (1, 4500, 20),
 ])
 def test_block_step_equals_two_pass_step(swe, solver, nx, ny):
     cur = [torch.empty((nx + 2) * (ny + 2), device="cuda") for _ in range(4)]
