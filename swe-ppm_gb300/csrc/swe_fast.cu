@@ -42,7 +42,7 @@
 namespace swegb {
 namespace fast {
 
-constexpr int kRing = 4;                          // column strips in flight per CTA (4 ran faster than 5, 6, 8)
+constexpr int kRing = 3;                          // column strips in flight per CTA (2048^2 step, 2 / 3 / 4: 36.6 / 33.9 / 34.2 us)
 constexpr int kHalo = 4;                          // staged rows below the tile (16-byte aligned start)
 constexpr int kSlice = kMaxTileRows + 2 * kHalo;  // floats per field of one strip
 constexpr int kSlotFloats = 4 * kSlice;           // h, hu, hv, b
@@ -853,7 +853,47 @@ __global__ void __launch_bounds__(kMaxTileRows / (2 * NP), MINB) fastStepKernel(
                     for (int r = 0; r < R; r++) nprev[r] = nxv[r];
                 }
                 // the block's rim: ghost pushes, edges to the block's own ghosts
+                bool rowsRim = rimWarp, slow = false;
                 if (RIMX && (xc == 1 || xc == nx)) {
+                    // the block's first or last column: outflow, wall and
+                    // neighbour ghosts inline, with the corners.  Through
+                    // rimCell, a call per row with its own chain of descriptor
+                    // loads, the CTAs with such a column ended last: 1252 ->
+                    // 1223 us for 33 steps of 2048^2 in 512^2 blocks, 7.5 ->
+                    // 6.2 us a step of 256^2; and without the calls here the
+                    // kernel needs 114 registers, not 128.
+                    const int side = xc == 1 ? 0 : 1;
+                    const int type = __ldg(&B.bnd[side]);
+                    slow = EDGES || nx == 1 || ny == 1 || (type != OUTFLOW && type != WALL && type != CONNECT_WITHIN_RANK);
+#pragma unroll
+                    for (int r = 0; r < R; r++) slow = slow || ((rimModes >> (3 * r)) & 7) >= 3;
+                    if (!slow) {
+                        const long long own = side ? (long long)(nx + 1) * P : 0;
+                        long long g = own;
+                        if (type == CONNECT_WITHIN_RANK) {
+                            const BlockDesc &N = f.d.blocks[__ldg(&B.nbr[side])];
+                            g = __ldg(&N.base) - base + (side ? 0 : (long long)(__ldg(&N.nx) + 1) * __ldg(&N.pitch));
+                        }
+#pragma unroll
+                        for (int r = 0; r < R; r++)
+                            if (r < nAct) {
+                                const int y = yA + r;
+                                const float hr = lanePick(hn[r / 2], r & 1), ur = lanePick(hun[r / 2], r & 1),
+                                            vr = lanePick(hvn[r / 2], r & 1);
+                                HO[g + y] = hr;
+                                HUO[g + y] = type == WALL ? -ur : ur;
+                                HVO[g + y] = vr;
+                                if (y == 1 || y == ny) {
+                                    const long long c = own + (y == 1 ? 0 : ny + 1);
+                                    HO[c] = hr;
+                                    HUO[c] = ur;
+                                    HVO[c] = vr;
+                                }
+                            }
+                    }
+                }
+                if (slow) {
+                    rowsRim = false;  // (rimCell pushes them)
 #pragma unroll
                     for (int r = 0; r < R; r++)
                         if (r < nAct)
@@ -861,7 +901,8 @@ __global__ void __launch_bounds__(kMaxTileRows / (2 * NP), MINB) fastStepKernel(
                                                           Hin, HUin, HVin, f.d.blocks, wu.block, xc, yA + r,
                                                           lanePick(hn[r / 2], r & 1), lanePick(hun[r / 2], r & 1),
                                                           lanePick(hvn[r / 2], r & 1)));
-                } else if (rimWarp) {
+                }
+                if (rowsRim) {
 #pragma unroll
                     for (int r = 0; r < R; r++) {
                         const int mode = (rimModes >> (3 * r)) & 7;
@@ -1001,10 +1042,11 @@ __global__ void __launch_bounds__(kMaxTileRows / (2 * NP), MINB) fastStepKernel(
 }
 
 /// Packed row pairs per thread of the step kernel and its resident CTAs per
-/// SM.  One pair at four CTAs of 128 threads: 128 registers, no spills, 16
+/// SM.  One pair at four CTAs of 128 threads: 114 registers, no spills, 16
 /// warps per SM.  The kernel is latency-bound, so warps count for more than
 /// instructions: two pairs issue 25% fewer instructions but need 216
-/// registers (8 warps per SM) and run 6% slower; one pair at five CTAs
+/// registers (8 warps per SM) and run 6% slower; one pair at five CTAs, or
+/// nine of 64 threads (five warps on a scheduler either way: 96 registers),
 /// spills.
 constexpr int kPairs = 1;
 constexpr int kMinCtas = 4;
