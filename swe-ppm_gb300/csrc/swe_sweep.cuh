@@ -539,7 +539,10 @@ __global__ void __launch_bounds__(GROUPED ? 1024 : kMaxTileRows, GROUPED ? 1 : 4
 
     // one segment: rows [wu.y0, wu.y0 + TY) x columns [wu.x0, wu.x1) of a block
     auto segment = [&](const WorkUnit wu, unsigned count, unsigned total) {
-        const BlockDesc B = d.blocks[wu.block];
+        // (by reference: the copy, on the stack, cost the split step 5%, the hybrid 6%;
+        // the four-team kernel alone runs 0.7% faster with it)
+        typename std::conditional<GROUPED, const BlockDesc, const BlockDesc &>::type B = d.blocks[wu.block];
+        const int nx = B.nx, ny = B.ny;
         // local time stepping: block k is dt group k, so the group's loads
         // need not wait for the block descriptor's
         GroupState *G = d.groups + (lts ? wu.block : B.group);
@@ -556,28 +559,28 @@ __global__ void __launch_bounds__(GROUPED ? 1024 : kMaxTileRows, GROUPED ? 1 : 4
         const int x0 = wu.x0, x1 = wu.x1, XC = x1 - x0;
         const int y0 = wu.y0;
         const int y = y0 + t;
-        const int yTop = min(y0 + TY - 1, B.ny);
+        const int yTop = min(y0 + TY - 1, ny);
         const bool active = y <= yTop;
         float smax = 0.f;
         float *__restrict__ HO = pick(d.h, cur ^ 1) + B.base;
         float *__restrict__ HUO = pick(d.hu, cur ^ 1) + B.base;
         float *__restrict__ HVO = pick(d.hv, cur ^ 1) + B.base;
-        const bool rimRow = y == 1 || y == B.ny;
+        const bool rimRow = y == 1 || y == ny;
         // a rim row (y == 1 or y == ny) pushes the ghost below / above each of
         // its cells every column, as pushGhosts does it: one store per field at
         // rimGhost + x * rimPitch (offsets from the block's base).  Outflow and
         // intra-rank sides copy the cell, a wall negates hv, the other types
         // (and every side under local time stepping) keep the ghost's value
-        // from the input buffer.  The block's first and last columns go
-        // through pushGhosts (corners).  Inline, because the CTA's barrier makes
+        // from the input buffer.  The block's first and last columns: see
+        // below.  Inline, because the CTA's barrier makes
         // every warp wait for the rim row's warp each column.
-        int rimMode = 0;  // 0: pushGhosts, 1: copy, 2: copy with -hv, 3: keep (local time stepping pushes none)
+        int rimMode = 0;  // 0: none (pushGhosts where ny is 1), 1: copy, 2: copy with -hv, 3: keep (local time stepping pushes none)
         long long rimGhost = 0;
         int rimPitch = 0;
-        if (UPDATE && rimRow && B.ny > 1 && !lts) {
+        if (UPDATE && rimRow && ny > 1 && !lts) {
             const int side = (y == 1) ? 2 : 3;
             const int type = B.bnd[side];
-            rimGhost = (side == 2) ? 0 : B.ny + 1;
+            rimGhost = (side == 2) ? 0 : ny + 1;
             rimPitch = B.pitch;
             if (type == OUTFLOW || type == WALL) {
                 rimMode = type == WALL ? 2 : 1;
@@ -686,9 +689,41 @@ __global__ void __launch_bounds__(GROUPED ? 1024 : kMaxTileRows, GROUPED ? 1 : 4
                             HVO[o] = hvn;
                             // no ghost pushes under local time stepping: the
                             // next check carries the ring over and rebuilds it
-                            if (!lts && (x - 1 == 1 || x - 1 == B.nx || rimRow)) {
-                                if (rimMode != 0 && x - 1 != 1 && x - 1 != B.nx) {
-                                    const long long g = rimGhost + (long long)(x - 1) * rimPitch;
+                            if (!lts && (x - 1 == 1 || x - 1 == nx || rimRow)) {
+                                // outflow, wall and neighbour ghosts (and the corners)
+                                // of the first and last column inline too: through
+                                // pushGhosts their CTAs ended the launch (2048^2 in
+                                // 512^2 blocks, exact step 65.2 -> 62.5 us; 1021 x
+                                // 2039 split step 33.1 -> 31.3)
+                                const int xc = x - 1;
+                                bool call = rimRow && rimMode == 0;
+                                if (xc == 1 || xc == nx) {
+                                    const int side = xc == 1 ? 0 : 1;
+                                    const int type = B.bnd[side];
+                                    call = call || nx == 1 || ny == 1 ||
+                                           (type != OUTFLOW && type != WALL && type != CONNECT_WITHIN_RANK);
+                                    if (!call) {
+                                        const long long own = side ? (long long)(nx + 1) * B.pitch : 0;
+                                        long long g = own;
+                                        if (type == CONNECT_WITHIN_RANK) {
+                                            const BlockDesc &N = d.blocks[B.nbr[side]];
+                                            g = N.base - B.base + (side ? 0 : (long long)(N.nx + 1) * N.pitch);
+                                        }
+                                        HO[g + y] = hn;
+                                        HUO[g + y] = type == WALL ? -hun : hun;
+                                        HVO[g + y] = hvn;
+                                        if (rimRow) {
+                                            const long long c = own + (y == 1 ? 0 : ny + 1);
+                                            HO[c] = hn;
+                                            HUO[c] = hun;
+                                            HVO[c] = hvn;
+                                        }
+                                    }
+                                }
+                                if (call) {
+                                    pushGhosts(d, B, cur ^ 1, P, xc, y, hn, hun, hvn);
+                                } else if (rimRow) {
+                                    const long long g = rimGhost + (long long)xc * rimPitch;
                                     if (rimMode == 3) {
                                         HO[g] = H[g];
                                         HUO[g] = HU[g];
@@ -698,8 +733,6 @@ __global__ void __launch_bounds__(GROUPED ? 1024 : kMaxTileRows, GROUPED ? 1 : 4
                                         HUO[g] = hun;
                                         HVO[g] = rimMode == 2 ? -hvn : hvn;
                                     }
-                                } else {
-                                    pushGhosts(d, B, cur ^ 1, P, x - 1, y, hn, hun, hvn);
                                 }
                             }
                         }
