@@ -85,7 +85,8 @@ typedef struct swe_gpu_desc {
     int solver;          /* SWE_SOLVER_* */
     int semantics;       /* SWE_SEMANTICS_* */
     int split_dt_mode;   /* SWE_SPLIT_DT_* (split semantics only) */
-    int tile_rows;       /* rows per CTA (multiple of 32, <= 256); 0 = default */
+    int tile_rows;       /* rows per CTA (multiple of 32, <= 256); 0 = default (256, or
+                            128 where that leaves clearly fewer rows idle) */
     int tile_cols;       /* max columns per work segment (<= 128 for the tile mapping); 0 = default */
     int device;          /* CUDA device ordinal */
     int kernel_variant;  /* reserved, must be 0 (the sweep kernels' one thread
@@ -206,8 +207,10 @@ int swe_gpu_get_max_timestep(swe_gpu_domain *dom, float *dt);
  * synchronisation */
 int swe_gpu_step(swe_gpu_domain *dom, int nsteps);
 /* the drivers' checkpoint loop `while (t < t_end) { step; t += dt; }`
- * (src/examples/swe_mpi.cpp:300-327) run on the device from a captured CUDA
- * graph; returns the executed steps and the float time reached */
+ * (src/examples/swe_mpi.cpp:300-327) run on the device in batches of steps (a
+ * captured CUDA graph of 16; a small domain's, up to 256 in one launch), a few
+ * batches ahead of the host; returns the executed steps and the float time
+ * reached */
 int swe_gpu_advance(swe_gpu_domain *dom, float t_end, int max_steps, int *steps_done, float *t_now);
 int swe_gpu_get_time(swe_gpu_domain *dom, float *t, int *steps);
 /* Update steps every block has executed (one entry per block; under local
@@ -275,7 +278,9 @@ int swe_gpu_set_time(swe_gpu_domain *dom, float t);
 
 /* waits for everything queued on the domain (steps, transfers, async downloads) */
 int swe_gpu_sync(swe_gpu_domain *dom);
-/* device-side status bits (bit 0: NaN wave speed); 0 when healthy */
+/* device-side status bits; 0 when healthy.  Bit 0: NaN wave speed, bit 1: a
+ * non-finite water height, bits 2 and 3: a bounded wait inside a kernel ran out
+ * (the fast step's copies, the meetings of a small domain's step) */
 int swe_gpu_status(swe_gpu_domain *dom, int *status);
 /* the CUDA stream the handle launches on (a cudaStream_t) */
 int swe_gpu_get_stream(swe_gpu_domain *dom, void **stream);

@@ -2,11 +2,11 @@
 //
 // One global time step of a group of blocks is two launches (plus a ghost
 // kernel only when the ghost ring is not already valid):
-//   sweepKernel<..., false>  speed pass: every edge's max wave speed, CTA max
+//   sweepKernel, UPDATE false  speed pass: every edge's max wave speed, CTA max
 //                    by warp shuffles, group max by atomicMax; the last
 //                    segment of the group turns it into maxTimestep
 //                    (src/blocks/SWE_DimensionalSplittingMpi.cpp:448-472)
-//   sweepKernel<..., true>   fused pass: solves every edge again, sums the net
+//   sweepKernel, UPDATE true   fused pass: solves every edge again, sums the net
 //                    updates per cell in registers and writes Q^{n+1} with the
 //                    dry clamp (src/blocks/SWE_DimensionalSplittingMpi.cpp:484-518)
 //                    or the split update (src/blocks/SWE_DimensionalSplitting.cpp:187-210),
@@ -26,7 +26,8 @@
 // solved from the previous column kept in registers, the y-edge (y|y+1) from
 // the neighbouring thread's cell in shared memory, and the tile's two boundary
 // y-edges per column are solved up front; a cell's update is finished one
-// column later, when its right edge is known.
+// column later, when its right edge is known.  GROUPED: four such teams share a
+// CTA that fills an SM, and keep pace.
 #pragma once
 
 #include <cstddef>
