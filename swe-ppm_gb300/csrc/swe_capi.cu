@@ -116,6 +116,7 @@ __device__ __forceinline__ void ghostCell(const DomainDev &d, const BlockDesc &B
 /// one mode 0 would write (the update pass pushed it): only hand it to the
 /// current state, as mode 0 does
 __global__ void ghostKernel(const DomainDev d, int mode) {
+    pdlWaitAndRelease();
     const bool bathymetry = mode == 1;
     const BlockDesc B = d.blocks[blockIdx.y];
     const GroupState *G = d.groups + B.group;
@@ -360,8 +361,7 @@ constexpr int kSmallSteps = 256;  // steps per launch of a small domain
 int enqueueGhost(swe_gpu_domain *D, int mode) {
     const int threads = mode == 3 ? 32 : 128;
     dim3 grid(mode == 3 ? 1 : (D->maxPerimeter + threads - 1) / threads, unsigned(D->blocks.size()));
-    ghostKernel<<<grid, threads, 0, D->stream>>>(D->dev, mode);
-    CUDA_TRY(cudaGetLastError());
+    CUDA_TRY(launchPdl(ghostKernel, grid, dim3(threads), D->stream, D->dev, mode));
     D->launches++;
     return SWE_GPU_OK;
 }

@@ -863,6 +863,11 @@ __device__ __forceinline__ void flushSpeed(const DomainDev &d, int group, float 
     smax = 0.f;
 }
 
+// The step's kernels wait for their predecessor on the device (programmatic
+// dependent launch; 2048^2 surrogate step 670 -> 660 us).  The augmented
+// solver's edge pass launches plainly: its registers are allocated to the last
+// one, and it gains nothing.
+
 /// Edge pass over a contiguous range of tiles per group of 128 threads (so the
 /// dt group changes rarely): the surrogate with the gate.  Groups whose time
 /// reached their target (or that sit the step out) are skipped, in this and
@@ -878,6 +883,7 @@ __global__ void __launch_bounds__(128 * kGroups, 2)
     __shared__ __align__(8) uint64_t mbar[kGroups];
     __shared__ uint32_t tslot;
     __shared__ __align__(16) float sHb[3 * kHid];  // halved hidden-layer biases
+    pdlWaitAndRelease();
     FwdGroup G = fwdBegin(image, smem, mbar, &tslot, sHb);
     const int t = G.t;
     bool ok = true;
@@ -965,6 +971,7 @@ __global__ void __launch_bounds__(128, 12) augEdgeKernel(const DomainDev d, cons
 /// maxTimestep of every group from the edge pass's max wave speed
 /// (src/blocks/SWE_DimensionalSplittingMpi.cpp:448-456)
 __global__ void surrogateDtKernel(const DomainDev d, int ngroups) {
+    pdlWaitAndRelease();
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= ngroups) return;
     GroupState *G = d.groups + g;
@@ -980,6 +987,7 @@ __global__ void surrogateDtKernel(const DomainDev d, int ngroups) {
 /// the unsplit cell update (src/blocks/SWE_DimensionalSplittingMpi.cpp:458-492)
 /// from the stored net updates: Q^{n+1} of interior cell (i, j) into the other buffer
 __global__ void surrogateApplyKernel(const DomainDev d, EdgeUpdates u) {
+    pdlWaitAndRelease();
     const BlockDesc B = d.blocks[blockIdx.y];
     GroupState *G = d.groups + B.group;
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1009,6 +1017,7 @@ __global__ void surrogateApplyKernel(const DomainDev d, EdgeUpdates u) {
 }
 
 __global__ void surrogateFinishKernel(const DomainDev d, int ngroups) {
+    pdlWaitAndRelease();
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= ngroups) return;
     GroupState *G = d.groups + g;
@@ -1429,7 +1438,8 @@ cudaError_t launchSurrogateEdges(const DomainDev &d, const swe_mlp *m, const Edg
     if (ntiles <= 0) return cudaSuccess;
     if (m) {
         const int groups = fwdGroups(ntiles, m->sms), grid = std::min((ntiles + groups - 1) / groups, m->sms * m->fwdBlocksPerSm);
-        surrogateEdgeKernel<<<grid, 128 * groups, fwdSmem(groups), s>>>(d, m->image, tiles, ntiles, u, used, m->err);
+        return launchPdlSmem(surrogateEdgeKernel, dim3(grid), dim3(128 * groups), size_t(fwdSmem(groups)), s, d, m->image, tiles,
+                             ntiles, u, used, m->err);
     } else {
         // the augmented solver alone: as many resident CTAs as registers allow
         // (latency hiding for its long dependency chains), looked up once per device
@@ -1445,24 +1455,21 @@ cudaError_t launchSurrogateEdges(const DomainDev &d, const swe_mlp *m, const Edg
         }
         const int grid = std::min(ntiles, smCount[dev] * perSm[dev]);
         augEdgeKernel<<<grid, 128, 0, s>>>(d, tiles, ntiles, u);
+        return cudaGetLastError();
     }
-    return cudaGetLastError();
 }
 
 cudaError_t launchSurrogateDt(const DomainDev &d, int ngroups, cudaStream_t s) {
-    surrogateDtKernel<<<(ngroups + 127) / 128, 128, 0, s>>>(d, ngroups);
-    return cudaGetLastError();
+    return launchPdl(surrogateDtKernel, dim3((ngroups + 127) / 128), dim3(128), s, d, ngroups);
 }
 
 cudaError_t launchSurrogateApply(const DomainDev &d, EdgeUpdates u, int nblocks, long long maxCells, cudaStream_t s) {
     const dim3 grid(unsigned((maxCells + 255) / 256), unsigned(nblocks));
-    surrogateApplyKernel<<<grid, 256, 0, s>>>(d, u);
-    return cudaGetLastError();
+    return launchPdl(surrogateApplyKernel, grid, dim3(256), s, d, u);
 }
 
 cudaError_t launchSurrogateFinish(const DomainDev &d, int ngroups, cudaStream_t s) {
-    surrogateFinishKernel<<<(ngroups + 127) / 128, 128, 0, s>>>(d, ngroups);
-    return cudaGetLastError();
+    return launchPdl(surrogateFinishKernel, dim3((ngroups + 127) / 128), dim3(128), s, d, ngroups);
 }
 
 cudaError_t launchLogEdges(const DomainDev &d, const EdgeTile *tiles, int ntiles, int stride, float *slots,
