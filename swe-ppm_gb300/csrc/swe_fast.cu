@@ -496,14 +496,27 @@ __global__ void __launch_bounds__(kMaxTileRows / (2 * NP), MINB) fastStepKernel(
         for (int q = 0; q < 4; q++)
             for (int i = t; i < kSlice; i += nth) ring[s * kSlotFloats + q * kSlice + i] = q == 0 ? 1.f : 0.f;
     // the partition and the block descriptors are written only when the
-    // domain is built: bring the first segment's into L1 before the wait
-    if (t == 0) {
-        const int s0 = f.ctaSeg[blockIdx.x];
-        if (s0 < f.ctaSeg[blockIdx.x + 1]) {
-            prefetchL1(&f.units[s0]);
-            prefetchL1(&f.d.blocks[f.units[s0].block]);
-        }
-    }
+    // domain is built: the first segment's are read before the wait (2048^2, 33
+    // steps: 1218 -> 1207 us; a prefetch into L1 before)
+    const int segBegin = f.ctaSeg[blockIdx.x], segEnd = f.ctaSeg[blockIdx.x + 1];
+    Unit wu{};
+    GroupState *G = nullptr;
+    unsigned P = 0u;
+    long long base = 0;
+    int nx = 0, ny = 0;
+    float bdx = 1.f, bdy = 1.f;
+    auto describe = [&](int seg) {
+        wu = f.units[seg];
+        const BlockDesc &B = f.d.blocks[wu.block];
+        G = f.d.groups + __ldg(&B.group);
+        P = unsigned(__ldg(&B.pitch));
+        base = __ldg(&B.base);
+        nx = __ldg(&B.nx);
+        ny = __ldg(&B.ny);
+        bdx = __ldg(&B.dx);
+        bdy = __ldg(&B.dy);
+    };
+    if (segBegin < segEnd) describe(segBegin);
     if (t == 0) {
         for (int s = 0; s < kRing; s++) {
             mbarInit(smemAddr(&mbar[s]), 1u);
@@ -520,16 +533,11 @@ __global__ void __launch_bounds__(kMaxTileRows / (2 * NP), MINB) fastStepKernel(
     pdlWaitAndRelease();
 
     const unsigned ringAddr = smemAddr(ring);
-    const int segEnd = f.ctaSeg[blockIdx.x + 1];
-    for (int seg = f.ctaSeg[blockIdx.x]; seg < segEnd; ++seg) {
-        const Unit wu = f.units[seg];
-        const BlockDesc &B = f.d.blocks[wu.block];
-        GroupState *G = f.d.groups + __ldg(&B.group);
+    for (int seg = segBegin; seg < segEnd; ++seg) {
+        if (seg > segBegin) describe(seg);
         if (!groupActive(G)) continue;
+        const BlockDesc &B = f.d.blocks[wu.block];
         const int cur = __ldg(&G->cur);
-        const unsigned P = unsigned(__ldg(&B.pitch));
-        const long long base = __ldg(&B.base);
-        const int nx = __ldg(&B.nx), ny = __ldg(&B.ny);
         const int x0 = wu.x0, x1 = wu.x1, XC = x1 - x0, ncol = XC + 2;  // columns x0-1 .. x1
         const int y0 = wu.y0, yTop = min(y0 + TY - 1, ny);
         const int rowStart = y0 - kHalo;
@@ -537,8 +545,8 @@ __global__ void __launch_bounds__(kMaxTileRows / (2 * NP), MINB) fastStepKernel(
         float2 dtdx, dtdy;
         {
             const float dt = __ldg(&G->dt);
-            dtdx = pk(__fdiv_rn(dt, __ldg(&B.dx)));
-            dtdy = pk(__fdiv_rn(dt, __ldg(&B.dy)));
+            dtdx = pk(__fdiv_rn(dt, bdx));
+            dtdy = pk(__fdiv_rn(dt, bdy));
         }
         const float *__restrict__ Hin = pick(f.d.h, cur);
         const float *__restrict__ HUin = pick(f.d.hu, cur);
@@ -861,7 +869,7 @@ __global__ void __launch_bounds__(kMaxTileRows / (2 * NP), MINB) fastStepKernel(
                     // loads, the CTAs with such a column ended last: 1252 ->
                     // 1223 us for 33 steps of 2048^2 in 512^2 blocks, 7.5 ->
                     // 6.2 us a step of 256^2; and without the calls here the
-                    // kernel needs 114 registers, not 128.
+                    // kernel needed 114 registers, not 128.
                     const int side = xc == 1 ? 0 : 1;
                     const int type = __ldg(&B.bnd[side]);
                     slow = EDGES || nx == 1 || ny == 1 || (type != OUTFLOW && type != WALL && type != CONNECT_WITHIN_RANK);
@@ -1042,7 +1050,7 @@ __global__ void __launch_bounds__(kMaxTileRows / (2 * NP), MINB) fastStepKernel(
 }
 
 /// Packed row pairs per thread of the step kernel and its resident CTAs per
-/// SM.  One pair at four CTAs of 128 threads: 114 registers, no spills, 16
+/// SM.  One pair at four CTAs of 128 threads: 122 registers, no spills, 16
 /// warps per SM.  The kernel is latency-bound, so warps count for more than
 /// instructions: two pairs issue 25% fewer instructions but need 216
 /// registers (8 warps per SM) and run 6% slower; one pair at five CTAs, or
