@@ -19,7 +19,7 @@
 // Every wait is bounded; one that runs out sets status bit 3 and leaves.
 //
 // Bound by the two meetings (about 1.5 us each) and the edges' latency, not by
-// bandwidth or issue.  256^2 hybrid step: 16.6 us as two passes, 7.7 us here.
+// bandwidth or issue.  256^2 hybrid step: 16.6 us as two passes, 7.1 us here.
 #include "swe_small.hpp"
 #include "swe_sweep.cuh"
 
@@ -56,6 +56,9 @@ __global__ void __launch_bounds__(kMaxTileRows, XC > 2 ? 3 : 4)
     const int t = threadIdx.x, TY = blockDim.x;
     const WorkUnit wu = units[blockIdx.x];
     const BlockDesc B = d.blocks[wu.block];
+    const int nx = B.nx, ny = B.ny;
+    const long long base = B.base;
+    const float dx = B.dx, dy = B.dy;
     GroupState *G = d.groups + B.group;
     if (!groupActive(G)) return;  // the whole group alike
     Sync *Y = sync + B.group;
@@ -69,10 +72,32 @@ __global__ void __launch_bounds__(kMaxTileRows, XC > 2 ? 3 : 4)
     unsigned seen = unsigned(*(volatile unsigned long long *)&Y->epoch >> 32);
 
     const int n = wu.x1 - wu.x0, x0 = wu.x0, y0 = wu.y0, y = y0 + t;
-    const int yTop = min(y0 + TY - 1, B.ny), last = yTop - y0;
+    const int yTop = min(y0 + TY - 1, ny), last = yTop - y0;
     const bool active = t <= last;
     const unsigned P = unsigned(B.pitch);
-    const float *BT = d.b + B.base;
+    const float *BT = d.b + base;
+
+    // a rim row's ghost: one store per field at rimGhost + x * rimPitch, as in
+    // the update pass (0: none, 1: copy, 2: copy with -hv, 3: keep); the first
+    // and last column's inline too.  (All through pushGhosts: 256^2 hybrid 7.36
+    // us a step, 7.07 so; with the descriptor by reference instead of copied a
+    // single step is 5% slower.)
+    const bool rimRow = active && (y == 1 || y == ny);
+    int rimMode = 0, rimPitch = int(P);
+    long long rimGhost = 0;
+    if (rimRow && ny > 1) {
+        const int side = (y == 1) ? 2 : 3, type = B.bnd[side];
+        rimGhost = (side == 2) ? 0 : ny + 1;
+        rimMode = 3;
+        if (type == OUTFLOW || type == WALL) {
+            rimMode = type == WALL ? 2 : 1;
+        } else if (type == CONNECT_WITHIN_RANK) {
+            const BlockDesc &N = d.blocks[B.nbr[side]];
+            rimMode = 1;
+            rimGhost = N.base - base + ((side == 2) ? N.ny + 1 : 0);
+            rimPitch = N.pitch;
+        }
+    }
 
     float qh[XC], qhu[XC], qhv[XC], qb[XC];
 #pragma unroll
@@ -81,9 +106,9 @@ __global__ void __launch_bounds__(kMaxTileRows, XC > 2 ? 3 : 4)
         qhu[c] = qhv[c] = qb[c] = 0.f;
         if (c < n && active) {
             const unsigned o = unsigned(x0 + c) * P + unsigned(y);
-            qh[c] = __ldcg(pick(d.h, cur) + B.base + o);
-            qhu[c] = __ldcg(pick(d.hu, cur) + B.base + o);
-            qhv[c] = __ldcg(pick(d.hv, cur) + B.base + o);
+            qh[c] = __ldcg(pick(d.h, cur) + base + o);
+            qhu[c] = __ldcg(pick(d.hu, cur) + base + o);
+            qhv[c] = __ldcg(pick(d.hv, cur) + base + o);
             qb[c] = __ldg(BT + o);
         }
     }
@@ -91,7 +116,7 @@ __global__ void __launch_bounds__(kMaxTileRows, XC > 2 ? 3 : 4)
     bool bad = false;
     int done = 0;
     while (done < nsteps && time < target) {
-        const float *H = pick(d.h, cur) + B.base, *HU = pick(d.hu, cur) + B.base, *HV = pick(d.hv, cur) + B.base;
+        const float *H = pick(d.h, cur) + base, *HU = pick(d.hu, cur) + base, *HV = pick(d.hv, cur) + base;
         // the cells across the segment's sides: left and right column of this
         // row, and (threads 0 .. 2n-1) one cell below or above
         float lh = 1.f, lhu = 0.f, lhv = 0.f, lb = 0.f, rh = 1.f, rhu = 0.f, rhv = 0.f, rb = 0.f;
@@ -194,8 +219,8 @@ __global__ void __launch_bounds__(kMaxTileRows, XC > 2 ? 3 : 4)
         }
         dt = sDt;
         // Q^{n+1}, as the update pass forms it
-        const float dtdx = dt / B.dx, dtdy = dt / B.dy;
-        float *HO = pick(d.h, cur ^ 1) + B.base, *HUO = pick(d.hu, cur ^ 1) + B.base, *HVO = pick(d.hv, cur ^ 1) + B.base;
+        const float dtdx = dt / dx, dtdy = dt / dy;
+        float *HO = pick(d.h, cur ^ 1) + base, *HUO = pick(d.hu, cur ^ 1) + base, *HVO = pick(d.hv, cur ^ 1) + base;
 #pragma unroll
         for (int c = 0; c < XC; c++) {
             if (c >= n || !active) break;
@@ -213,7 +238,44 @@ __global__ void __launch_bounds__(kMaxTileRows, XC > 2 ? 3 : 4)
             HO[o] = hn;
             HUO[o] = hun;
             HVO[o] = hvn;
-            if (x == 1 || x == B.nx || y == 1 || y == B.ny) pushGhosts(d, B, cur ^ 1, P, x, y, hn, hun, hvn);
+            if (x == 1 || x == nx || rimRow) {
+                bool call = rimRow && rimMode == 0;
+                if (x == 1 || x == nx) {
+                    const int side = x == 1 ? 0 : 1, type = B.bnd[side];
+                    call = call || nx == 1 || ny == 1 || (type != OUTFLOW && type != WALL && type != CONNECT_WITHIN_RANK);
+                    if (!call) {
+                        const long long own = side ? (long long)(nx + 1) * P : 0;
+                        long long g = own;
+                        if (type == CONNECT_WITHIN_RANK) {
+                            const BlockDesc &N = d.blocks[B.nbr[side]];
+                            g = N.base - base + (side ? 0 : (long long)(N.nx + 1) * N.pitch);
+                        }
+                        HO[g + y] = hn;
+                        HUO[g + y] = type == WALL ? -hun : hun;
+                        HVO[g + y] = hvn;
+                        if (rimRow) {  // the corner
+                            const long long k = own + (y == 1 ? 0 : ny + 1);
+                            HO[k] = hn;
+                            HUO[k] = hun;
+                            HVO[k] = hvn;
+                        }
+                    }
+                }
+                if (call) {
+                    pushGhosts(d, B, cur ^ 1, P, x, y, hn, hun, hvn);
+                } else if (rimRow) {
+                    const long long g = rimGhost + (long long)x * rimPitch;
+                    if (rimMode == 3) {
+                        HO[g] = __ldcg(H + g);
+                        HUO[g] = __ldcg(HU + g);
+                        HVO[g] = __ldcg(HV + g);
+                    } else {
+                        HO[g] = hn;
+                        HUO[g] = hun;
+                        HVO[g] = rimMode == 2 ? -hvn : hvn;
+                    }
+                }
+            }
             qh[c] = hn;
             qhu[c] = hun;
             qhv[c] = hvn;

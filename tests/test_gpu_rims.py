@@ -12,13 +12,14 @@ pytestmark = pytest.mark.gpu
 OUT, WALL, INFLOW, CONNECT, PASSIVE = 0, 1, 2, 3, 5
 
 
+@pytest.mark.parametrize("speed_pass", [0, 1])  # small domains: their own kernel, and the two passes
 @pytest.mark.parametrize("semantics,nx_cols,ny_rows", [
     (0, [1], [1]), (0, [5], [1]), (0, [1], [70]), (0, [40], [259]), (0, [33, 20], [64, 31]), (0, [700, 520], [256, 512]),
     (1, [1], [1]), (1, [1], [70]), (1, [40], [259]),
 ])
 @pytest.mark.parametrize("solver", ["HLLE", "HYBRID"])
 @pytest.mark.parametrize("boundary", [[OUT, WALL, WALL, OUT], [WALL, OUT, PASSIVE, WALL], [INFLOW, WALL, OUT, CONNECT]])
-def test_pushed_ring_equals_recomputed_ring(swe, solver, semantics, nx_cols, ny_rows, boundary):
+def test_pushed_ring_equals_recomputed_ring(swe, solver, semantics, nx_cols, ny_rows, boundary, speed_pass):
     n = sum((x + 2) * (y + 2) for x in nx_cols for y in ny_rows)
     r = np.random.default_rng(n)
     st = [10 + r.random(n), r.random(n) - 0.5, r.random(n) - 0.5, -10 + 0.1 * r.random(n)]
@@ -26,7 +27,7 @@ def test_pushed_ring_equals_recomputed_ring(swe, solver, semantics, nx_cols, ny_
 
     def make(state):
         D = swe.Domain(nx_cols, ny_rows, 10.0, 12.0, boundary=boundary, solver=getattr(swe, solver), semantics=semantics,
-                       speed_pass=1)
+                       speed_pass=speed_pass)
         D.upload(*state)
         return D
 
