@@ -1097,7 +1097,7 @@ int buildDomain(const std::vector<BlockSpec> &spec, const DomainOptions &o, swe_
     D->edgeBuffered = D->solver == SOLVER_AUGRIE && D->semantics == SEM_UNSPLIT && !D->lts &&
                       o.speedPass == 0;
     if (D->edgeBuffered) {
-        D->stepTiles = mlp::buildStepTiles(D->blocks);
+        D->stepTiles = mlp::buildStepTiles(D->blocks, mlp::edgeRanges());
         ok = ok && cudaMalloc(&D->edgeBuf, 8 * bytes) == cudaSuccess;
         ok = ok && cudaMalloc(&D->dUsed, sizeof(unsigned long long)) == cudaSuccess;
         ok = ok && cudaMalloc(&D->dStepTiles, sizeof(mlp::EdgeTile) * std::max<size_t>(1, D->stepTiles.size())) == cudaSuccess;
@@ -2197,7 +2197,7 @@ static int ensureEdgeTiles(swe_gpu_domain *D) {
 }
 static int ensureStepTiles(swe_gpu_domain *D) {
     if (D->dStepTiles) return SWE_GPU_OK;
-    D->stepTiles = mlp::buildStepTiles(D->blocks);
+    D->stepTiles = mlp::buildStepTiles(D->blocks, mlp::edgeRanges());
     return uploadTiles(D->stepTiles, &D->dStepTiles);
 }
 

@@ -1433,6 +1433,22 @@ int swe_mlp_gemm_check(int mode, int w1, int w2, const float *x, const float *y,
 namespace swegb {
 namespace mlp {
 
+int edgeRanges() {
+    // the augmented solver alone: as many resident CTAs as registers allow
+    // (latency hiding for its long dependency chains), looked up once per device
+    static int perSm[64] = {0}, smCount[64] = {0};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64) dev = 0;
+    if (!perSm[dev]) {
+        cudaDeviceGetAttribute(&smCount[dev], cudaDevAttrMultiProcessorCount, dev);
+        int occ = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, augEdgeKernel, 128, 0);
+        perSm[dev] = std::max(1, occ);
+    }
+    return smCount[dev] * perSm[dev];
+}
+
 cudaError_t launchSurrogateEdges(const DomainDev &d, const swe_mlp *m, const EdgeTile *tiles, int ntiles, EdgeUpdates u,
                                  unsigned long long *used, cudaStream_t s) {
     if (ntiles <= 0) return cudaSuccess;
@@ -1441,19 +1457,7 @@ cudaError_t launchSurrogateEdges(const DomainDev &d, const swe_mlp *m, const Edg
         return launchPdlSmem(surrogateEdgeKernel, dim3(grid), dim3(128 * groups), size_t(fwdSmem(groups)), s, d, m->image, tiles,
                              ntiles, u, used, m->err);
     } else {
-        // the augmented solver alone: as many resident CTAs as registers allow
-        // (latency hiding for its long dependency chains), looked up once per device
-        static int perSm[64] = {0}, smCount[64] = {0};
-        int dev = 0;
-        cudaGetDevice(&dev);
-        if (dev < 0 || dev >= 64) dev = 0;
-        if (!perSm[dev]) {
-            cudaDeviceGetAttribute(&smCount[dev], cudaDevAttrMultiProcessorCount, dev);
-            int occ = 0;
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, augEdgeKernel, 128, 0);
-            perSm[dev] = std::max(1, occ);
-        }
-        const int grid = std::min(ntiles, smCount[dev] * perSm[dev]);
+        const int grid = std::min(ntiles, edgeRanges());
         augEdgeKernel<<<grid, 128, 0, s>>>(d, tiles, ntiles, u);
         return cudaGetLastError();
     }
