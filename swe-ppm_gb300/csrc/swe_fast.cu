@@ -118,21 +118,19 @@ __device__ __forceinline__ FQ makeFQ(float h, float hn, float eta, float ih, flo
     q.h = h;
     q.hn = hn;
     q.eta = eta;
-    q.u = __fmul_rn(hn, ih);
+    q.u = hn * ih;
     q.sq = sq;
-    q.m = __fmul_rn(hn, q.u);
-    q.lo = __fsub_rn(q.u, c);
-    q.hi = __fadd_rn(q.u, c);
+    q.m = hn * q.u;
+    q.lo = q.u - c;
+    q.hi = q.u + c;
     return q;
 }
 
-/// the same from raw values (one reciprocal square root).  Every operation of
-/// the single-edge forms is rounded by itself, as the packed ones are: an edge
-/// that two lanes solve, one in each form, gives both the same bits.
+/// the same from raw values (one reciprocal square root)
 __device__ __forceinline__ FQ rawFQ(float h, float hn, float b) {
     const float r = aRsqrt(h);
-    const float sq = __fmul_rn(h, r);
-    return makeFQ(h, hn, __fadd_rn(h, b), __fmul_rn(r, r), sq, __fmul_rn(kSqrtG, sq));
+    const float sq = h * r;
+    return makeFQ(h, hn, h + b, r * r, sq, kSqrtG * sq);
 }
 
 __device__ __forceinline__ void routeFast(float s, float zh, float zhu, float &hL, float &hR, float &huL, float &huR) {
@@ -160,32 +158,32 @@ __device__ __forceinline__ void routeFast(float s, float zh, float zhu, float &h
 template <int S, bool GENERAL>
 __device__ __forceinline__ void waves(const FQ &L, const FQ &R, float &aL, float &aR, float &auL, float &auR,
                                       float &sub) {
-    const float rs = aRcp(__fadd_rn(L.sq, R.sq));
-    const float uRoe = __fmul_rn(fmaf(L.u, L.sq, __fmul_rn(R.u, R.sq)), rs);
-    const float ghs = __fmul_rn(kHalfG, __fadd_rn(L.h, R.h));
+    const float rs = aRcp(L.sq + R.sq);
+    const float uRoe = fmaf(L.u, L.sq, R.u * R.sq) * rs;
+    const float ghs = kHalfG * (L.h + R.h);
     const float cRoe = aSqrt(ghs);
-    float s1 = __fsub_rn(uRoe, cRoe), s2 = __fadd_rn(uRoe, cRoe);
+    float s1 = uRoe - cRoe, s2 = uRoe + cRoe;
     if (S == SOLVER_HLLE) {
         s1 = fminf(L.lo, s1);
         s2 = fmaxf(R.hi, s2);
     }
-    const float df1 = __fsub_rn(R.hn, L.hn);
-    const float df2 = fmaf(ghs, __fsub_rn(R.eta, L.eta), __fsub_rn(R.m, L.m));
-    const float rd = aRcp(__fsub_rn(s2, s1));
-    const float b1 = __fmul_rn(fmaf(s2, df1, -df2), rd);
-    const float b2 = __fmul_rn(fmaf(-s1, df1, df2), rd);
+    const float df1 = R.hn - L.hn;
+    const float df2 = fmaf(ghs, R.eta - L.eta, R.m - L.m);
+    const float rd = aRcp(s2 - s1);
+    const float b1 = fmaf(s2, df1, -df2) * rd;
+    const float b2 = fmaf(-s1, df1, df2) * rd;
     if (GENERAL) {
         aL = 0.f;
         aR = 0.f;
         auL = 0.f;
         auR = 0.f;
-        routeFast(s1, b1, __fmul_rn(b1, s1), aL, aR, auL, auR);
-        routeFast(s2, b2, __fmul_rn(b2, s2), aL, aR, auL, auR);
+        routeFast(s1, b1, b1 * s1, aL, aR, auL, auR);
+        routeFast(s2, b2, b2 * s2, aL, aR, auL, auR);
     } else {
         aL = b1;
-        auL = __fmul_rn(b1, s1);
+        auL = b1 * s1;
         aR = b2;
-        auR = __fmul_rn(b2, s2);
+        auR = b2 * s2;
         sub = fminf(sub, fminf(-s1, s2));
     }
 }
