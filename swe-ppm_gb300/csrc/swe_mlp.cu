@@ -494,7 +494,8 @@ __global__ void __launch_bounds__(128, 1) trainKernel(const uint8_t *image, Edge
     uint8_t *const act = smem + kTrA1;  // A1, A2, A3
     // what does not depend on the batch before -- the constant operands, the
     // TMEM columns, the first tile's edges -- comes before the wait for its
-    // Adam step, the weights after it
+    // Adam step, the weights after it.  (The first batch of an order, whose
+    // predecessor writes that order, is launched without a head start: trainBatch.)
     for (int i = t; i < kOnesBytes / 4; i += blockDim.x) reinterpret_cast<uint32_t *>(sOnes)[i] = 0x3F803F80u;  // BF16 1.0
     for (int i = t; i < (kTrEnd - kTrDZ4) / 4; i += blockDim.x) reinterpret_cast<uint32_t *>(sDZ4)[i] = 0u;
     if (t == 0) tc::mbarInit(&mbar, 1);
@@ -1139,11 +1140,21 @@ struct swe_mlp {
         MLP_TRY(cudaGetLastError());
         return SWE_GPU_OK;
     }
-    /// gradient (and optionally an Adam step) of the batch; loss sum to *lossDst (device)
-    int trainBatch(const EdgeBatch &b, float invN, float lr, float *gradDst, float *lossDst) {
+    /// gradient (and optionally an Adam step) of the batch; loss sum to *lossDst (device).
+    /// afterBatch: the launch before it is the Adam step of another batch of the
+    /// same edges in the same order.  Only then may the training kernel start
+    /// before that launch is over: it reads its first edges ahead of its wait,
+    /// and for any other batch the copies or the shuffle that write them (and
+    /// the order they are taken in) may still be in flight.
+    int trainBatch(const EdgeBatch &b, float invN, float lr, float *gradDst, float *lossDst, bool afterBatch) {
         const int ntiles = (b.count + kTile - 1) / kTile;
         const int grid = std::max(1, std::min(ntiles, sms));
-        MLP_TRY(launchPdlSmem(trainKernel, dim3(grid), dim3(128), kTrSmem, nullptr, image, b, invN, partials, err));
+        if (afterBatch) {
+            MLP_TRY(launchPdlSmem(trainKernel, dim3(grid), dim3(128), kTrSmem, nullptr, image, b, invN, partials, err));
+        } else {
+            trainKernel<<<grid, 128, kTrSmem>>>(image, b, invN, partials, err);
+            MLP_TRY(cudaGetLastError());
+        }
         float bc1 = 1.f, bc2 = 1.f;
         if (lr > 0.f) {
             adamSteps++;
@@ -1324,7 +1335,7 @@ int swe_mlp_loss_grad(swe_mlp *m, int n, const float *edges, const float *target
     MLP_TRY(cudaMemcpy(m->buf, edges, size_t(6) * n * sizeof(float), cudaMemcpyHostToDevice));
     MLP_TRY(cudaMemcpy(m->buf + size_t(6) * n, targets, size_t(4) * n * sizeof(float), cudaMemcpyHostToDevice));
     EdgeBatch b{m->buf, m->buf + size_t(6) * n, nullptr, n, 0, n};
-    if ((rc = m->trainBatch(b, 1.f / float(n), 0.f, m->grad, m->grad + kNParams))) return rc;
+    if ((rc = m->trainBatch(b, 1.f / float(n), 0.f, m->grad, m->grad + kNParams, false))) return rc;
     MLP_TRY(cudaMemcpy(grad, m->grad, kNParams * sizeof(float), cudaMemcpyDeviceToHost));
     float sum = 0.f;
     MLP_TRY(cudaMemcpy(&sum, m->grad + kNParams, sizeof(float), cudaMemcpyDeviceToHost));
@@ -1369,7 +1380,8 @@ int swe_mlp_train(swe_mlp *m, int n, const float *edges, const float *targets, i
         for (int k = 0; k < nb; k++) {
             const int off = k * batch, cnt = std::min(batch, n - off);
             EdgeBatch b{m->buf, m->buf + size_t(6) * n, m->perm, n, off, cnt};
-            if ((rc = m->trainBatch(b, 1.f / float(cnt), lr, nullptr, m->losses + size_t(ep) * nb + k))) return rc;
+            if ((rc = m->trainBatch(b, 1.f / float(cnt), lr, nullptr, m->losses + size_t(ep) * nb + k, k > 0)))
+                return rc;
         }
     }
     std::vector<float> bl(size_t(nb) * epochs);
