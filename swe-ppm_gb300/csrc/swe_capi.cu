@@ -272,8 +272,6 @@ struct swe_gpu_domain {
     int maxCols = 0;              // max nx+2 over blocks
     cudaGraphExec_t graph = nullptr;
     int graphSteps = 0;
-    // small domains, in the place of the graph: decided by the first swe_gpu_advance
-    bool smallPrimed = false, smallRing = false, smallStale = false;
     // swe_gpu_advance: the groups' states at its start and after each batch of
     // steps in flight (pinned), the events that mark their copies, and the
     // clock and dt it saw last
@@ -1634,21 +1632,26 @@ int swe_gpu_advance(swe_gpu_domain *dom, float t_end, int max_steps, int *steps_
         int rc0 = enqueueFastPrologue(dom);
         if (rc0) return rc0;
     }
-    // A small domain's steps need no graph, many go out in one launch (256^2,
-    // 17 steps: 158 -> 152 us a call, 128 steps 1056 -> 963).  Whether batches of 16 and more set a stale ghost ring
-    // first is decided at the first call, as the capture below does it.
-    const bool direct = dom->smallCols > 0;
-    if (direct && !dom->smallPrimed) {
-        dom->smallPrimed = true;
-        dom->smallRing = dom->smallStale = !dom->ghostsValid;
+    // Steps start on a valid ghost ring; one that an upload left stale is set
+    // here, before any step is queued and outside the graph, whose replays then
+    // need no ghost kernel whenever it was captured.
+    if (!dom->ghostsValid && max_steps > 0) {
+        int rc0 = enqueueGhost(dom, 0);
+        if (rc0) return rc0;
         dom->ghostsValid = true;
     }
+    // A small domain's steps need no graph, many go out in one launch (256^2,
+    // 17 steps: 158 -> 152 us a call, 128 steps 1056 -> 963).
+    const bool direct = dom->smallCols > 0;
     if (!direct && !dom->graph) {  // capture `batch` steps once; replays are identical
+        const bool ring = dom->ghostsValid;
+        dom->ghostsValid = true;  // (for the steps that are captured)
         cudaGraph_t g;
         CUDA_TRY(cudaStreamBeginCapture(dom->stream, cudaStreamCaptureModeThreadLocal));
         int rc = SWE_GPU_OK;
         const long long before = dom->launches;
         rc = enqueueSteps(dom, batch);
+        dom->ghostsValid = ring;
         cudaError_t e = cudaStreamEndCapture(dom->stream, &g);
         dom->graphKernels = dom->launches - before;  // captured, not launched
         dom->launches = before;
@@ -1694,15 +1697,7 @@ int swe_gpu_advance(swe_gpu_domain *dom, float t_end, int max_steps, int *steps_
                (ahead == 0 || double(seenTime) + double(seenDt) * (queued - seenQueued) < double(t_end))) {
             if (ahead > 0 && !(seenDt > 0.f)) break;
             const int n = std::min(max_steps - queued, direct ? kSmallSteps : dom->graphSteps);
-            if (direct && n >= batch) {
-                if (dom->smallRing && (dom->smallStale || !dom->ghostsValid)) {
-                    rc = enqueueGhost(dom, 0);
-                    if (rc) return rc;
-                    dom->smallStale = false;
-                }
-                rc = enqueueSmall(dom, n);
-                if (rc) return rc;
-            } else if (!direct && n == dom->graphSteps) {
+            if (!direct && n == dom->graphSteps) {
                 CUDA_TRY(cudaGraphLaunch(dom->graph, dom->stream));
                 dom->launches += dom->graphKernels;
             } else {
@@ -1935,7 +1930,6 @@ int swe_gpu_retile(swe_gpu_domain *dom, int tile_rows, int tile_cols) {
     if (dom->graph) cudaGraphExecDestroy(dom->graph);
     if (dom->ltsGraph) cudaGraphExecDestroy(dom->ltsGraph);
     dom->graph = nullptr;
-    dom->smallPrimed = false;
     dom->ltsGraph = nullptr;
     return SWE_GPU_OK;
 }
