@@ -16,14 +16,17 @@
 //  - Each thread owns two consecutive rows of a tile, computed as packed
 //    pairs (f32x2 add / mul / fma), and marches along x.  The x-edge (x-1|x)
 //    uses the previous column kept in registers, the y-edges the thread's
-//    own rows and the staged rows above and below them.  Every lane solves
-//    its bottom y-edge itself, although the lane below has solved it as its
-//    top one: the warp issues it for lane 0 anyway, and without the branch
-//    around lane 0 and the shuffle after it the edge runs between the others
-//    (2048^2, back to back: 37.4 -> 34.8 us a step, with the masks of partial
-//    tiles as selects, not branches; warps in flight and latency bound the kernel).
-//    Where a warp solves its edges again (dry cells, supercritical edges),
-//    only lane 0 does the bottom one and the shuffle gives the others theirs.
+//    own rows and the staged rows above and below them.  A lane's bottom
+//    y-edge is the top one of the lane below, and it takes that lane's
+//    solution by a shuffle, so that both sides of an edge get one solution.
+//    Lane 0, which has no lane below, solves it itself; so does every lane,
+//    in vain: the warp issues it for lane 0 anyway, and without a branch
+//    around it the edge runs between the others (33 steps of 2048^2: 1306 ->
+//    1248 us when the branch went, with the masks of partial tiles as
+//    selects).  Keeping the lane's own instead of the shuffled one is 1.2%
+//    faster (1209 against 1224 us), but the two forms round apart here and
+//    there, and a warp that solves edges again (dry cells, supercritical
+//    edges) has to shuffle all the same.
 //  - The next step's maximum wave speed (computeNumericalFluxes :391-456 on
 //    Q^{n+1}) is evaluated while Q^{n+1} is produced: edges between two cells
 //    of the segment as soon as both exist, edges to a ghost from the boundary
@@ -713,6 +716,13 @@ __global__ void __launch_bounds__(kMaxTileRows / (2 * NP), MINB) fastStepKernel(
                 }
             }
             float lowRh = 0.f, lowRhv = 0.f, subLow = 3.0e38f;
+            // what this lane's first row gets from its bottom edge: the lane
+            // below's solution of it (lane 0: its own)
+            auto fromBelow = [&]() {
+                const float pH = __shfl_up_sync(FULL, aRy[NP - 1].y, 1), pHV = __shfl_up_sync(FULL, auRy[NP - 1].y, 1);
+                lowRh = lane == 0 ? lowRh : pH;
+                lowRhv = lane == 0 ? lowRhv : pHV;
+            };
             if (YCOL) {
 #pragma unroll
                 for (int q = 0; q < NP; q++)
@@ -721,6 +731,7 @@ __global__ void __launch_bounds__(kMaxTileRows / (2 * NP), MINB) fastStepKernel(
                 minh = fminf(minh, up.h);
                 float dl, dlv;
                 waves<S, false>(low, laneX(cy[0]), dl, lowRh, dlv, lowRhv, subLow);
+                fromBelow();
             }
             // C. a lane with a dry cell or an edge that is not subsonic solves
             // its edges again in full (rare: shorelines, fronts)
@@ -758,14 +769,7 @@ __global__ void __launch_bounds__(kMaxTileRows / (2 * NP), MINB) fastStepKernel(
                             }
                         }
                     }
-                    if (YCOL) {  // the lane below has solved the other lanes' bottom edges
-                        const float pH = __shfl_up_sync(FULL, aRy[NP - 1].y, 1);
-                        const float pHV = __shfl_up_sync(FULL, auRy[NP - 1].y, 1);
-                        if (lane != 0) {
-                            lowRh = pH;
-                            lowRhv = pHV;
-                        }
-                    }
+                    if (YCOL) fromBelow();
                 }
             }
             // D. cells (x-1, y): Q^{n+1} with the dry clamp, and their part
