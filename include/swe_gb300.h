@@ -204,7 +204,12 @@ int swe_gpu_update_unknowns(swe_gpu_domain *dom, float dt);
 int swe_gpu_get_max_timestep(swe_gpu_domain *dom, float *dt);
 
 /* `nsteps` fused steps (ghosts + fluxes + update) queued on the stream; no host
- * synchronisation */
+ * synchronisation.  A small domain's exact unsplit steps (all its CTAs fit on
+ * the device at once) go out in cooperative launches, here and in
+ * swe_gpu_advance: such a launch starts when there is room for all of its
+ * CTAs, so a kernel of the caller's that holds SMs must not wait on the device
+ * for the step to finish.  On a stream of a green context (a part of the SMs),
+ * and where the launch is refused, the steps take two launches each instead */
 int swe_gpu_step(swe_gpu_domain *dom, int nsteps);
 /* the drivers' checkpoint loop `while (t < t_end) { step; t += dt; }`
  * (src/examples/swe_mpi.cpp:300-327) run on the device in batches of steps (a
@@ -317,7 +322,9 @@ int swe_gpu_solve_edges(int solver, long long n, const float *hL, const float *h
  * looks the array's device address up (cudaGetSymbolAddress); make that first
  * call before any stream capture.  A call that meets a CUDA error forgets the
  * address, so the next call looks it up again (after a cudaDeviceReset).  Every call on a device shares the array and
- * clears it when it starts: calls that overlap on the GPU race. */
+ * clears it when it starts: calls that overlap on the GPU race.  A block whose
+ * CTAs all fit on the device at once takes its unsplit step in a cooperative
+ * launch, under the conditions given at swe_gpu_step. */
 int swe_gpu_step_block_noalloc(int solver, int semantics, int nx, int ny, float dx, float dy, const int *boundary4,
                                int ld, float *h, float *hu, float *hv, const float *b, float *h_out, float *hu_out,
                                float *hv_out, float *dt_out, void *stream);

@@ -312,9 +312,11 @@ struct swe_gpu_domain {
     // the speed and the update pass
     bool edgeBuffered = false;
     // small domains (swe_small.cu): several steps per launch, smallCols (0: the
-    // domain is not small) columns per CTA of tileRows rows
+    // domain is not small) columns per CTA of tileRows rows, on streams that
+    // can have the whole device
     int speedPassArg = 0;
     int smallCols = 0;
+    bool wholeDevice = true;
     std::vector<WorkUnit> unitsS;
     std::vector<small::Sync> syncInit;  // one per dt group
     WorkUnit *dUnitsS = nullptr;
@@ -500,20 +502,34 @@ int enqueueStep(swe_gpu_domain *D) {
     return enqueueUpdate(D);
 }
 
-/// `n` steps of a small domain, in launches of at most kSmallSteps
+/// `n` steps of a small domain, in launches of at most kSmallSteps, or by the
+/// passes where the CTAs cannot be resident together after all
 int enqueueSmall(swe_gpu_domain *D, int n) {
-    for (int done = 0; done < n; done += kSmallSteps) {
-        CUDA_TRY(small::launch(D->dev, D->dUnitsS, int(D->unitsS.size()), D->dSync, std::min(n - done, kSmallSteps),
-                               D->smallCols, D->tileRows, D->stream));
+    for (int done = 0; done < n;) {
+        const int now = std::min(n - done, kSmallSteps);
+        const cudaError_t e = small::launch(D->dev, D->dUnitsS, int(D->unitsS.size()), D->dSync, now, D->smallCols, D->tileRows,
+                                            D->stream);
+        if (small::refused(e)) {
+            for (; done < n; done++) {
+                int rc = enqueueStep(D);
+                if (rc) return rc;
+            }
+            break;
+        }
+        CUDA_TRY(e);
         D->launches++;
         D->ghostsValid = true;
+        done += now;
     }
     return SWE_GPU_OK;
 }
 
+/// whether the domain's steps go out several to a launch
+bool stepsSmall(const swe_gpu_domain *D) { return D->smallCols > 0 && D->wholeDevice; }
+
 /// `n` steps
 int enqueueSteps(swe_gpu_domain *D, int n) {
-    if (!D->smallCols) {
+    if (!stepsSmall(D)) {
         for (int i = 0; i < n; i++) {
             int rc = enqueueStep(D);
             if (rc) return rc;
@@ -1159,6 +1175,7 @@ int buildDomain(const std::vector<BlockSpec> &spec, const DomainOptions &o, swe_
         }
     }
     buildSmallPlan(D);
+    D->wholeDevice = small::wholeDevice(D->stream);
     if (const int rcP = uploadPlan(D)) {
         freeDomain(D);
         return rcP;
@@ -1642,7 +1659,7 @@ int swe_gpu_advance(swe_gpu_domain *dom, float t_end, int max_steps, int *steps_
     }
     // A small domain's steps need no graph, many go out in one launch (256^2,
     // 17 steps: 158 -> 152 us a call, 128 steps 1056 -> 963).
-    const bool direct = dom->smallCols > 0;
+    const bool direct = stepsSmall(dom);
     if (!direct && !dom->graph) {  // capture `batch` steps once; replays are identical
         const bool ring = dom->ghostsValid;
         dom->ghostsValid = true;  // (for the steps that are captured)
@@ -2152,6 +2169,7 @@ int swe_gpu_set_stream(swe_gpu_domain *dom, void *stream) {
     CUDA_TRY(cudaSetDevice(dom->device));
     CUDA_TRY(cudaStreamSynchronize(dom->stream));
     dom->stream = stream ? static_cast<cudaStream_t>(stream) : dom->ownStream;
+    dom->wholeDevice = small::wholeDevice(dom->stream);
     return SWE_GPU_OK;
 }
 
@@ -2419,7 +2437,12 @@ extern "C" int swe_gpu_step_block_noalloc(int solver, int semantics, int nx, int
     // launch less and every edge solved once: 128^2 HLLE 20.6 -> 15.5 us, 424 x
     // 26 augmented 34.9 -> 22.5, 1200 x 256 f-wave 29.7 -> 23.7 (a call each).
     // It gains up to its limit, the CTAs that are resident at once.
-    const int smallCols = semantics == SWE_SEMANTICS_UNSPLIT ? noallocSmallCols(device, solver, tileRows, rowTiles, nx) : 0;
+    // (Not on a stream that has only a part of the device; and where the launch
+    // is refused, the passes run on its units.)
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const int smallCols = semantics == SWE_SEMANTICS_UNSPLIT && small::wholeDevice(s)
+                              ? noallocSmallCols(device, solver, tileRows, rowTiles, nx)
+                              : 0;
     const int cols = smallCols ? smallCols : tileCols;
     const long long nunits = rowTiles * ((nx + cols - 1) / cols);
     NoAllocScratch *scr = nullptr;
@@ -2452,7 +2475,6 @@ extern "C" int swe_gpu_step_block_noalloc(int solver, int semantics, int nx, int
     d.solver = solver;
     d.semantics = semantics;
     d.splitDtMode = SPLIT_DT_MAX;
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
 
     // any CUDA error drops the device's cached scratch address, so a call
     // after the context was torn down (cudaDeviceReset) looks it up again
@@ -2468,10 +2490,13 @@ extern "C" int swe_gpu_step_block_noalloc(int solver, int semantics, int nx, int
     noallocSetupKernel<<<unsigned((setupItems + threads - 1) / threads), threads, 0, s>>>(scr, d, B, tileRows, cols,
                                                                                        int(nunits));
     if ((rc = check(cudaGetLastError(), "set-up kernel"))) return rc;
+    bool passes = smallCols == 0;
     if (smallCols) {
-        rc = check(small::launch(d, scr->units, int(nunits), &scr->sync, 1, smallCols, tileRows, s), "step");
-        if (rc) return rc;
-    } else {
+        const cudaError_t e = small::launch(d, scr->units, int(nunits), &scr->sync, 1, smallCols, tileRows, s);
+        passes = small::refused(e);
+        if (!passes && (rc = check(e, "step"))) return rc;
+    }
+    if (passes) {
         if ((rc = check(launchSpeed(d, int(nunits), tileRows, s, false), "speed pass"))) return rc;
         if ((rc = check(launchUpdate(d, int(nunits), tileRows, 1, s), "update pass"))) return rc;
     }

@@ -20,6 +20,8 @@
 //
 // Bound by the two meetings (about 1.5 us each) and the edges' latency, not by
 // bandwidth or issue.  256^2 hybrid step: 16.6 us as two passes, 7.1 us here.
+#include <cudaTypedefs.h>
+
 #include "swe_small.hpp"
 #include "swe_sweep.cuh"
 
@@ -342,6 +344,23 @@ int capacity(int solver, int cols, int threads) {
     return coop ? sms * occ : 0;
 }
 
+bool wholeDevice(cudaStream_t s) {
+    // (looked up once; a driver without it has no green contexts)
+    static const PFN_cuStreamGetGreenCtx_v12040 ask = [] {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        const cudaError_t e = cudaGetDriverEntryPointByVersion("cuStreamGetGreenCtx", &f, 12040, cudaEnableDefault, &q);
+        if (e != cudaSuccess) cudaGetLastError();
+        return reinterpret_cast<PFN_cuStreamGetGreenCtx_v12040>(e == cudaSuccess && q == cudaDriverEntryPointSuccess ? f : nullptr);
+    }();
+    CUgreenCtx green = nullptr;
+    return !ask || (ask(s, &green) == CUDA_SUCCESS && !green);
+}
+
+bool refused(cudaError_t e) {
+    return e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorLaunchOutOfResources || e == cudaErrorNotSupported;
+}
+
 cudaError_t launch(const DomainDev &d, const WorkUnit *units, int nunits, Sync *sync, int nsteps, int cols, int threads,
                    cudaStream_t s) {
     cudaLaunchConfig_t cfg = {};
@@ -354,7 +373,8 @@ cudaError_t launch(const DomainDev &d, const WorkUnit *units, int nunits, Sync *
     cfg.attrs = at;
     cfg.numAttrs = 1;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, pickKernel(d.solver, cols), d, units, sync, nsteps);
-    return e != cudaSuccess ? e : cudaGetLastError();
+    const cudaError_t last = cudaGetLastError();  // (clears a refusal's)
+    return e != cudaSuccess ? e : last;
 }
 
 } // namespace small

@@ -25,6 +25,16 @@ constexpr int kMaxCols = 4;  // most columns of a CTA's segment
 /// resident at once on the current device; 0 when it cannot launch them together
 int capacity(int solver, int cols, int threads);
 
+/// Whether work on the stream can have the whole device, as capacity() takes it
+/// to.  The SMs of a green context are a part of it, and a cooperative launch
+/// that does not fit that part is not refused but never starts: such streams
+/// (and any that cannot be told) take the passes, which need no CTAs together.
+bool wholeDevice(cudaStream_t s);
+
+/// Whether launch() failed because its CTAs cannot be resident together (a
+/// context with fewer SMs than the device says): the passes run all the same
+bool refused(cudaError_t e);
+
 /// up to nsteps unsplit steps of every group that has not reached its target
 /// (fewer once it has); units[i] is CTA i's segment of at most `cols` columns
 cudaError_t launch(const DomainDev &d, const WorkUnit *units, int nunits, Sync *sync, int nsteps, int cols, int threads,
