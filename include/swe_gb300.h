@@ -285,7 +285,9 @@ int swe_gpu_set_time(swe_gpu_domain *dom, float t);
 int swe_gpu_sync(swe_gpu_domain *dom);
 /* device-side status bits; 0 when healthy.  Bit 0: NaN wave speed, bit 1: a
  * non-finite water height, bits 2 and 3: a bounded wait inside a kernel ran out
- * (the fast step's copies, the meetings of a small domain's step) */
+ * (the fast step's copies, the meetings of a small domain's step).  After bit
+ * 3 the group's state is not to be used and swe_gpu_step and swe_gpu_advance
+ * leave it as it is: create the handle anew */
 int swe_gpu_status(swe_gpu_domain *dom, int *status);
 /* the CUDA stream the handle launches on (a cudaStream_t) */
 int swe_gpu_get_stream(swe_gpu_domain *dom, void **stream);
@@ -324,7 +326,9 @@ int swe_gpu_solve_edges(int solver, long long n, const float *hL, const float *h
  * address, so the next call looks it up again (after a cudaDeviceReset).  Every call on a device shares the array and
  * clears it when it starts: calls that overlap on the GPU race.  A block whose
  * CTAs all fit on the device at once takes its unsplit step in a cooperative
- * launch, under the conditions given at swe_gpu_step. */
+ * launch, under the conditions given at swe_gpu_step.  If its CTAs do not meet
+ * (a bounded wait runs out), the call has no status to say so: dt_out is NaN,
+ * and h_out is NaN wherever it was not computed. */
 int swe_gpu_step_block_noalloc(int solver, int semantics, int nx, int ny, float dx, float dy, const int *boundary4,
                                int ld, float *h, float *hu, float *hv, const float *b, float *h_out, float *hu_out,
                                float *hv_out, float *dt_out, void *stream);

@@ -566,6 +566,14 @@ int readGroups(swe_gpu_domain *D, std::vector<GroupState> &g) {
     return SWE_GPU_OK;
 }
 
+/// error of a run whose groups' status bits are `status`
+int checkStatus(int status) {
+    if (!status) return SWE_GPU_OK;
+    return fail(SWE_GPU_ERR_DEVICE, "device status 0x%x%s%s%s%s", status, status & 1 ? " (NaN wave speed)" : "",
+                status & 2 ? " (non-finite water height)" : "", status & 4 ? " (a wait of the fast step ran out)" : "",
+                status & 8 ? " (a meeting of a small domain's step ran out)" : "");
+}
+
 int setTargets(swe_gpu_domain *D, float target) {
     setTargetsKernel<<<(D->ngroups + 255) / 256, 256, 0, D->stream>>>(D->dGroups, D->ngroups, target);
     CUDA_TRY(cudaGetLastError());
@@ -1741,7 +1749,8 @@ int swe_gpu_advance(swe_gpu_domain *dom, float t_end, int max_steps, int *steps_
         seenDt = 0.f;
         for (int i = 0; i < ng; i++) {
             done = std::max(done, g[i].steps - start[i].steps);
-            all = all && !(g[i].time < t_end);
+            // (a group whose meeting ran out steps no more)
+            all = all && (!(g[i].time < t_end) || (g[i].status & 8));
             if (g[i].time < seenTime) {
                 seenTime = g[i].time;
                 seenDt = g[i].dt;
@@ -1761,10 +1770,7 @@ int swe_gpu_advance(swe_gpu_domain *dom, float t_end, int max_steps, int *steps_
         status |= g[i].status;
     }
     if (t_now) *t_now = tmin;
-    if (dom->smallCols && (status & 8))  // a wait ran out: the meeting points start afresh
-        CUDA_TRY(cudaMemcpy(dom->dSync, dom->syncInit.data(), sizeof(small::Sync) * dom->syncInit.size(), cudaMemcpyHostToDevice));
-    if (status) return fail(SWE_GPU_ERR_DEVICE, "device status 0x%x (NaN wave speed)", status);
-    return SWE_GPU_OK;
+    return checkStatus(status);
 }
 
 int swe_gpu_lts_advance(swe_gpu_domain *dom, float t_end, int max_iterations, int *intervals_done, float *t_now) {
@@ -1842,7 +1848,7 @@ int swe_gpu_lts_advance(swe_gpu_domain *dom, float t_end, int max_iterations, in
     if (rc) return rc;
     int status = 0;
     for (const GroupState &s : g) status |= s.status;
-    if (status) return fail(SWE_GPU_ERR_DEVICE, "device status 0x%x", status);
+    if ((rc = checkStatus(status))) return rc;
     if (c.t < t_end && c.iterations - startIterations >= max_iterations)
         return SWE_GPU_INCOMPLETE;  // the iteration budget ran out first
     return SWE_GPU_OK;

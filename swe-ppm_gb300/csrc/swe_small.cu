@@ -16,7 +16,8 @@
 //     load;
 //   - the update with the dry clamp (:484-518), the ghost pushes of the block's
 //     rim, and a second meeting before the next step reads the new cells.
-// Every wait is bounded; one that runs out sets status bit 3 and leaves.
+// Every wait is bounded; a CTA whose wait runs out leaves (giveUp), and no later
+// launch steps the group again.
 //
 // Bound by the two meetings (about 1.5 us each) and the edges' latency, not by
 // bandwidth or issue.  256^2 hybrid step: 16.6 us as two passes, 7.1 us here.
@@ -45,6 +46,17 @@ __device__ __forceinline__ void publishEpoch(Sync *y, unsigned number, float dt)
     asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(&y->epoch), "l"(e) : "memory");
 }
 
+/// A CTA leaves without its meeting: status bit 3, and for a caller who reads no
+/// status (the allocation-free call has none) dt and the depths that this CTA
+/// was to write are NaN.
+static __device__ __noinline__ void giveUp(GroupState *G, float *H, unsigned pitch, int columns) {
+    if (threadIdx.x == 0) {
+        atomicOr(&G->status, 8);
+        atomicExch(&G->dt, NAN);
+    }
+    for (int c = 0; c < columns; c++) H[size_t(c) * pitch] = NAN;
+}
+
 template <int S, int XC>
 __global__ void __launch_bounds__(kMaxTileRows, XC > 2 ? 3 : 4)
     smallStepKernel(const DomainDev d, const WorkUnit *units, Sync *sync, int nsteps) {
@@ -54,6 +66,8 @@ __global__ void __launch_bounds__(kMaxTileRows, XC > 2 ? 3 : 4)
     __shared__ float sRed[kMaxTileRows / 32];
     __shared__ float sDt;
     __shared__ int sGo;
+    __shared__ int sDead;           // an earlier meeting ran out: the meeting point is not to be used
+    __shared__ unsigned sDtBefore;  // the dt that the leader replaces at the end
 
     const int t = threadIdx.x, TY = blockDim.x;
     const WorkUnit wu = units[blockIdx.x];
@@ -68,6 +82,10 @@ __global__ void __launch_bounds__(kMaxTileRows, XC > 2 ? 3 : 4)
     float time = G->time;
     const float target = G->target;
     const int need = Y->ctas;
+    if (t == 0) {  // (thread 0's alone, here to leave the registers to the edges)
+        sDead = G->status & 8;
+        sDtBefore = __float_as_uint(G->dt);
+    }
     const bool leader = Y->first == int(blockIdx.x);
     // the meetings' number before this launch's first one: it cannot move
     // before every CTA of the group, this one included, has arrived
@@ -195,8 +213,10 @@ __global__ void __launch_bounds__(kMaxTileRows, XC > 2 ? 3 : 4)
         // the group's maximum speed, dt
         const float m = blockReduceMax(smax, sRed);
         if (t == 0) {
-            atomicMax(&Y->speed, __float_as_uint(m));
-            if (arriveAcqRel(&Y->count, 1u) + 1u == unsigned(need)) {
+            if (!sDead) atomicMax(&Y->speed, __float_as_uint(m));
+            if (sDead) {
+                sGo = 0;
+            } else if (arriveAcqRel(&Y->count, 1u) + 1u == unsigned(need)) {
                 const float s = __uint_as_float(__ldcg(&Y->speed));
                 const BlockDesc &F = d.blocks[G->firstBlock];
                 dt = timestepFromSpeed(s, F.dx, F.dy, SEM_UNSPLIT);
@@ -216,7 +236,7 @@ __global__ void __launch_bounds__(kMaxTileRows, XC > 2 ? 3 : 4)
         __syncthreads();
         seen++;
         if (!sGo) {
-            if (t == 0) atomicOr(&G->status, 8);
+            giveUp(G, pick(d.h, cur ^ 1) + base + size_t(x0) * P + y, P, active ? n : 0);
             return;
         }
         dt = sDt;
@@ -299,14 +319,15 @@ __global__ void __launch_bounds__(kMaxTileRows, XC > 2 ? 3 : 4)
             __syncthreads();
             seen++;
             if (!sGo) {
-                if (t == 0) atomicOr(&G->status, 8);
+                giveUp(G, pick(d.h, cur) + base + size_t(x0) * P + y, P, active ? n : 0);
                 return;
             }
         }
     }
     if (__syncthreads_or(bad) && t == 0) atomicOr(&G->status, 2);
     if (leader && t == 0) {  // (every CTA of the group has read the state above before the first meeting)
-        G->dt = dt;
+        // (dt stays NaN where a CTA of the group has given up)
+        atomicCAS(reinterpret_cast<unsigned *>(&G->dt), sDtBefore, __float_as_uint(dt));
         G->time = time;
         G->steps += done;
         G->cur = cur;
