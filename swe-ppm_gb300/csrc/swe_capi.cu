@@ -681,8 +681,11 @@ long long paddedRows(const std::vector<BlockDesc> &blocks, int TY) {
 /// Default tile height: 256 rows, unless 128-row tiles idle at least 5% fewer
 /// rows.  Where both fill alike, taller tiles solve fewer boundary edges twice
 /// and win by 2-9% (4096^2 as 4 x 4 blocks, fast / exact step: 125 / 231 us
-/// against 128 / 252); partial tiles turn that round (6 x 6 blocks of 300^2,
-/// 1.71 against 1.28 rows per cell: 72 / 87 us against 65 / 75).
+/// against 128 / 252).  One block of 4 M cells, HLLE, us a step with 128 against
+/// 256 rows, by the idle rows saved: 10%: exact 64.1 / 67.2, fast 48.9 / 57.3; 8%:
+/// 64.4 / 66.9, 51.5 / 56.8; 7%: 65.1 / 64.5, 33.6 / 56.0; 4%: 65.6 / 64.4, 34.3 /
+/// 54.1.  So the exact step breaks even near 7%, and the fast one gains wherever
+/// the taller tiles alone are partial; the line lies between.
 int defaultTileRows(const std::vector<BlockDesc> &blocks) {
     return paddedRows(blocks, 128) * 20 <= paddedRows(blocks, 256) * 19 ? 128 : 256;
 }
@@ -697,10 +700,12 @@ int tileRowsFor(const swe_gpu_domain *D, int arg) {
 /// CTA), else 32 where runs would pass 64 columns and 5% or more of the tiles'
 /// rows are idle.  Equal runs of columns are then unequal work (a run through
 /// a partial tile ends early), and short segments, dealt to CTAs as they
-/// finish, even it out: 128 dam breaks of 64..1024 rows, 637 -> 414 us a fast
-/// step, 702 -> 556 us an exact one (with the tile height above).  Full tiles
-/// gain nothing from it (4096^2: 125 -> 139 us a fast step), and local time
-/// stepping deals its segments out on the device.
+/// finish, even it out.  48 dam breaks of some 500 rows in 256-row tiles, us a
+/// step with one run against 32 columns, by the idle rows: 9%: exact 372 / 360,
+/// fast 356 / 296; 4.5%: 383 / 373, 353 / 288; 1%: 394 / 385, 357 / 289; none: 399 /
+/// 385, 203 / 213.  The line keeps full tiles, where the fast step loses by it
+/// (4096^2: 125 -> 139 us), well on the other side.  Local time stepping deals
+/// its segments out on the device.
 int segmentCap(const swe_gpu_domain *D, int TY, int arg, long long total, long long workers) {
     if (arg > 0) return arg;
     long long cells = 0;
@@ -899,18 +904,16 @@ int uploadFastPlan(swe_gpu_domain *D) {
 /// Small domains: exact unsplit step with the default segment length, where
 /// segments of 1, 2 or 4 columns cover the domain with CTAs that are resident
 /// together (4 per SM of 256 rows up to 2 columns, 3 at 4).  Step times against
-/// the passes' (us, f-wave and HLLE / hybrid / augmented solver): 256^2 7.2 / 7.7
-/// / 12 against 25 / 17 / 16, 512^2 11 / 11 / - against 24 / 20 / -, 640^2 14 /
-/// 15 / - against 25 / 28 / -.  The augmented solver's edges bound it sooner: at
-/// 2 columns it loses (400^2: 28 against 24).
+/// the passes' (us, f-wave and HLLE / hybrid / augmented solver): 256^2 6.9 / 7.2
+/// / 9.4 against 23.3 / 12.3 / 14.4, 400^2 8.4 / 8.7 / - against 22.4 / 15.6 / -,
+/// 640^2 13.1 / 13.8 / - against 22.5 / 22.9 / -.
 void buildSmallPlan(swe_gpu_domain *D) {
     D->smallCols = 0;
     D->unitsS.clear();
     D->syncInit.clear();
     if (D->fast || D->lts || D->semantics != SEM_UNSPLIT || D->speedPassArg != 0 || D->tileColsArg > 0) return;
     const int TY = D->tileRows;
-    const int most = D->solver == SOLVER_AUGRIE ? 1 : small::kMaxCols;
-    for (int cols = 1; cols <= most; cols *= 2) {
+    for (int cols = 1; cols <= small::maxCols(D->solver); cols *= 2) {
         long long n = 0;
         for (const BlockDesc &B : D->blocks) n += (long long)((B.ny + TY - 1) / TY) * ((B.nx + cols - 1) / cols);
         if (n > small::capacity(D->solver, cols, TY)) continue;

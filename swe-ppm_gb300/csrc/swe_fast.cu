@@ -1052,7 +1052,7 @@ __global__ void __launch_bounds__(kMaxTileRows / (2 * NP), MINB) fastStepKernel(
 }
 
 /// Packed row pairs per thread of the step kernel and its resident CTAs per
-/// SM.  One pair at four CTAs of 128 threads: 122 registers, no spills, 16
+/// SM.  One pair at four CTAs of 128 threads: 120 registers (f-wave 124), no spills, 16
 /// warps per SM.  The kernel is latency-bound, so warps count for more than
 /// instructions: two pairs issue 25% fewer instructions but need 216
 /// registers (8 warps per SM) and run 6% slower; one pair at five CTAs, or

@@ -78,7 +78,9 @@ constexpr int fwdSmem(int groups) { return kFwdAct + groups * kActBytes; }
 constexpr int kFwdSmem = fwdSmem(kGroups);
 constexpr uint32_t kFwdCols = 64;
 /// groups per CTA for a number of tiles: 4 once every SM has work for them, else
-/// 2 or 1, so that tiles spread over the SMs before they share one
+/// 2 or 1, so that tiles spread over the SMs before they share one.  A surrogate
+/// step on 152 SMs, us with 1 / 2 / 4 groups: 146 tiles 17.9 / 18.3 / 20.5, 154: 19.9 /
+/// 19.0 / 21.1, 299: 21.0 / 20.1 / 22.0, 307: 26.9 / 22.3 / 21.9, 2407: 61.8 / 45.7 / 39.4
 inline int fwdGroups(int ntiles, int sms) { return ntiles > 2 * sms ? kGroups : ntiles > sms ? 2 : 1; }
 // training kernel: shared memory ...
 constexpr int kTrOnes = kImageSmem, kTrX0 = kTrOnes + kOnesBytes, kTrA1 = kTrX0 + kX0Bytes, kTrA2 = kTrA1 + kActBytes,

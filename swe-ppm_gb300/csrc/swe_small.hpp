@@ -20,9 +20,15 @@ struct __align__(128) Sync {
 };
 
 constexpr int kMaxCols = 4;  // most columns of a CTA's segment
+/// ... of a solver's.  The augmented one's edges bound a CTA, and at two columns
+/// it lost to the passes when the line was drawn (400^2: 28 us a step against
+/// 24); with its edges as they are now, two columns take 13.8 us there and the
+/// passes 17.5
+constexpr int maxCols(int solver) { return solver == SOLVER_AUGRIE ? 1 : kMaxCols; }
 
-/// CTAs of `threads` rows and up to `cols` columns (1, 2 or 4) that are
-/// resident at once on the current device; 0 when it cannot launch them together
+/// CTAs of `threads` rows and up to `cols` columns (1, 2 or 4, at most
+/// maxCols(solver)) that are resident at once on the current device; 0 when it
+/// cannot launch them together
 int capacity(int solver, int cols, int threads);
 
 /// Whether work on the stream can have the whole device, as capacity() takes it
